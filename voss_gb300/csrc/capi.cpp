@@ -451,17 +451,13 @@ extern "C" int voss_primes_in_range_with_limit(uint64_t a, uint64_t b, uint64_t 
     if (b < a) return VOSS_OK;
     vg::Engine& E = vg::Engine::for_current_device();
     std::lock_guard<std::mutex> g(E.mu);
-    std::vector<uint64_t> v = vg::primes_in_range(E, a, b, max_count);
-    if (v.size() > max_count) {
+    vg::PrimeList v = vg::primes_in_range(E, a, b, max_count);
+    if (v.over) {
       set_err("Range contains more primes than max_count");
       return VOSS_ERR_OUT_OF_MEMORY;
     }
-    if (v.empty()) return VOSS_OK;
-    auto* p = (uint64_t*)malloc(v.size() * sizeof(uint64_t));
-    if (!p) { set_err("host malloc failed"); return VOSS_ERR_OUT_OF_MEMORY; }
-    std::memcpy(p, v.data(), v.size() * sizeof(uint64_t));
-    *out_array = p;
-    *out_count = v.size();
+    *out_count = v.n;
+    *out_array = v.take();
     return VOSS_OK;
   }, VOSS_ERR_CUDA);
 }
@@ -567,14 +563,14 @@ extern "C" int voss_primes_nth(uint64_t n, uint64_t* out) {
     if (c >= n) {                       // p_n <= est: the (c - n + 1)-th largest prime <= est
       const uint64_t lo = est > span ? est - span : 0;
       for (uint64_t lo2 = lo;; lo2 = lo2 > span ? lo2 - span : 0) {
-        std::vector<uint64_t> v = vg::primes_in_range(E, lo2, est, ~0ull >> 1);
-        if (v.size() >= c - n + 1) { *out = v[v.size() - (c - n + 1)]; return VOSS_OK; }
+        const vg::PrimeList v = vg::primes_in_range(E, lo2, est, ~0ull >> 1);
+        if (v.n >= c - n + 1) { *out = v.p[v.n - (c - n + 1)]; return VOSS_OK; }
         if (lo2 == 0) break;
       }
     } else {                            // p_n > est: the (n - c)-th prime after est
       for (uint64_t hi = est + span;; hi += span) {
-        std::vector<uint64_t> v = vg::primes_in_range(E, est + 1, hi, ~0ull >> 1);
-        if (v.size() >= n - c) { *out = v[n - c - 1]; return VOSS_OK; }
+        const vg::PrimeList v = vg::primes_in_range(E, est + 1, hi, ~0ull >> 1);
+        if (v.n >= n - c) { *out = v.p[n - c - 1]; return VOSS_OK; }
       }
     }
     set_err("internal: could not locate the n-th prime");

@@ -534,7 +534,7 @@ void Plan::load_requests(uint32_t n, const uint64_t* a, const uint64_t* b, uint3
   if (flags & kFlagBitmap) {
     if (n != 1) throw Error(VOSS_ERR_INTERNAL, "bitmap output needs exactly one range");
     const uint64_t words = (host_reqs[0].k_hi - host_reqs[0].k_lo + 3) / 4 + 1;
-    bitmap.reserve(words * 4);
+    bitmap.reserve_ahead(words * 4);
   }
   if (!cap_req) {
     bucket.reserve(4 * std::max<uint64_t>(bucket_entries, 1));

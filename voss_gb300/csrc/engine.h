@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <memory>
 #include <mutex>
@@ -33,6 +34,9 @@ struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
   void reserve(size_t n);
+  // reserve(n) with room for somewhat larger sizes to come (an eighth, at most
+  // 32 MB), for buffers whose size follows a caller's range.
+  void reserve_ahead(size_t n) { if (n > bytes || !ptr) reserve(n + std::min<size_t>(n / 8, 32u << 20)); }
   void release();
   template <class T> T* as() const { return static_cast<T*>(ptr); }
   ~DevBuf() { release(); }
@@ -207,6 +211,8 @@ struct TuneEntry {
   uint32_t pad;
 };
 
+struct BitmapWork;      // goldbach.cu
+
 class Engine {
  public:
   static Engine& for_current_device();
@@ -235,6 +241,10 @@ class Engine {
 
   // Scratch plan reused by the synchronous entry points.
   Plan scratch;
+  // Buffers of the synchronous calls that read a wheel bitmap (in_range,
+  // Sophie Germain, Goldbach), kept between calls up to a bound (guarded by
+  // mu like scratch).
+  std::shared_ptr<BitmapWork> bitmap_work;
 
   void ensure_table(uint64_t pmax);
   uint32_t primes_below_sq(uint64_t b) const;   // table primes p with p*p < b

@@ -17,8 +17,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
+#include <exception>
 #include <memory>
+#include <new>
 #include <vector>
 
 #include "attr_cache.h"
@@ -386,7 +389,9 @@ __global__ void extract_write_kernel(const uint32_t* __restrict__ wb, uint64_t n
 const uint32_t* sieve_bitmap(Engine& E, Plan& plan, uint64_t a, uint64_t b_excl, uint64_t* nwords) {
   plan.eng = &E;
   plan.device = E.device;
-  plan.load(1, &a, &b_excl, kFlagBitmap);
+  plan.timed = false;
+  const uint32_t count_only = 0;          // the readers need no gap scan
+  plan.load(1, &a, &b_excl, kFlagBitmap, &count_only);
   plan.launch(E.stream);
   *nwords = (plan.host_reqs[0].k_hi - plan.host_reqs[0].k_lo + 3) / 4;
   return plan.bitmap.as<uint32_t>();
@@ -415,15 +420,21 @@ struct GoldbachPlan {
   bool want_minp = false;
 };
 
-GoldbachPlan* goldbach_plan_create(Engine& E, uint64_t N) {
-  std::unique_ptr<GoldbachPlan> g(new GoldbachPlan());
+// Size g for N, keeping what it holds.
+static void goldbach_plan_set(GoldbachPlan* g, Engine& E, uint64_t N) {
   g->eng = &E;
   g->N = N;
-  const std::vector<uint32_t> op = odd_primes_below(65535);
-  g->oddp.reserve(op.size() * 4);
-  check_cuda(cudaMemcpy(g->oddp.ptr, op.data(), op.size() * 4, cudaMemcpyHostToDevice), "odd primes");
+  g->sieve.nreq = 0;                      // its request is loaded at the next launch
+  if (!g->oddp.ptr) {
+    const std::vector<uint32_t> op = odd_primes_below(65535);
+    DevBuf d;                             // kept only once it is filled
+    d.reserve(op.size() * 4);
+    check_cuda(cudaMemcpy(d.ptr, op.data(), op.size() * 4, cudaMemcpyHostToDevice), "odd primes");
+    std::swap(g->oddp.ptr, d.ptr);
+    std::swap(g->oddp.bytes, d.bytes);
+  }
   g->odd_words = (N / 2 + 1 + 31) / 32 + 2;
-  g->odd.reserve((g->odd_words + 2 * kGbPad) * 4);
+  g->odd.reserve_ahead((g->odd_words + 2 * kGbPad) * 4);
   g->hist.reserve(sizeof(unsigned long long) * kGoldbachHistBins);
   g->scalars.reserve(64);
   g->ce_cap = 1024;
@@ -435,16 +446,59 @@ GoldbachPlan* goldbach_plan_create(Engine& E, uint64_t N) {
     per_sm = 1;
   g->grid = (uint32_t)std::min<uint64_t>(g->ntiles, (uint64_t)E.sm_count * per_sm);
   g->sieve.eng = &E;
+  g->sieve.device = E.device;
   g->sieve.timed = false;
+}
+
+GoldbachPlan* goldbach_plan_create(Engine& E, uint64_t N) {
+  std::unique_ptr<GoldbachPlan> g(new GoldbachPlan());
+  goldbach_plan_set(g.get(), E, N);
   return g.release();
 }
+
+// What the synchronous calls keep on the device between them: a call that
+// allocates and frees its bitmap pays more for that than for its kernels
+// (Goldbach to 10^9: 0.6 of 2.3 ms; Sophie Germain to 10^7: most of 0.1 ms).
+// Above kKeepBytes everything is given back at the end of the call.
+constexpr size_t kKeepBytes = 256u << 20;
+
+struct BitmapWork {
+  Plan sieve;                    // in_range, Sophie Germain
+  DevBuf counts, offsets, primes, total;
+  GoldbachPlan gb;
+  size_t bytes() const {
+    return sieve.bitmap.bytes + counts.bytes + offsets.bytes + primes.bytes + gb.sieve.bitmap.bytes +
+           gb.odd.bytes + gb.minp.bytes + gb.ce.bytes;
+  }
+};
+
+namespace {
+
+// The engine's kept buffers for one call (the caller holds the engine's lock).
+class KeptWork {
+ public:
+  explicit KeptWork(Engine& e) : E(e), thrown(std::uncaught_exceptions()) {
+    if (!E.bitmap_work) E.bitmap_work = std::make_shared<BitmapWork>();
+  }
+  // a call that failed leaves nothing half built behind
+  ~KeptWork() {
+    if (std::uncaught_exceptions() > thrown || E.bitmap_work->bytes() > kKeepBytes) E.bitmap_work.reset();
+  }
+  BitmapWork* operator->() const { return E.bitmap_work.get(); }
+ private:
+  Engine& E;
+  int thrown;
+};
+
+}  // namespace
 
 void goldbach_plan_launch(GoldbachPlan* g, cudaStream_t s) {
   Engine& E = *g->eng;
   // wheel bitmap of [0, N] (sieve kernel on the same stream)
   {
     uint64_t a = 0, b = g->N + 1;
-    if (!g->sieve.nreq || g->sieve.host_reqs[0].b != b) g->sieve.load(1, &a, &b, kFlagBitmap);
+    const uint32_t count_only = 0;
+    if (!g->sieve.nreq || g->sieve.host_reqs[0].b != b) g->sieve.load(1, &a, &b, kFlagBitmap, &count_only);
     g->sieve.launch(s);
   }
   const uint32_t* wb = g->sieve.bitmap.as<uint32_t>();
@@ -517,12 +571,12 @@ void goldbach_plan_free(GoldbachPlan* g) { delete g; }
 
 GoldbachResult goldbach_run(Engine& E, uint64_t N, uint32_t* minp_host, uint64_t max_ce,
                             float* kernel_ms) {
-  std::unique_ptr<GoldbachPlan> g(goldbach_plan_create(E, N));
+  KeptWork work(E);
+  GoldbachPlan* const g = &work->gb;
+  goldbach_plan_set(g, E, N);
   const uint64_t nn = (N - 4) / 2 + 1;
-  if (minp_host) {
-    g->want_minp = true;
-    g->minp.reserve(4 * nn);
-  }
+  g->want_minp = minp_host != nullptr;
+  if (minp_host) g->minp.reserve_ahead(4 * nn);
   g->ce_cap = std::max<uint64_t>(std::min<uint64_t>(max_ce, 1ull << 24), 1);
   g->ce.reserve(8 * g->ce_cap);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -531,10 +585,10 @@ GoldbachResult goldbach_run(Engine& E, uint64_t N, uint32_t* minp_host, uint64_t
     check_cuda(cudaEventCreate(&e1), "event");
     check_cuda(cudaEventRecord(e0, E.stream), "event");
   }
-  goldbach_plan_launch(g.get(), E.stream);
+  goldbach_plan_launch(g, E.stream);
   if (kernel_ms) check_cuda(cudaEventRecord(e1, E.stream), "event");
   GoldbachResult r;
-  goldbach_plan_fetch(g.get(), &r, E.stream);
+  goldbach_plan_fetch(g, &r, E.stream);
   if (kernel_ms) {
     check_cuda(cudaEventElapsedTime(kernel_ms, e0, e1), "event");
     cudaEventDestroy(e0);
@@ -551,10 +605,10 @@ GoldbachResult goldbach_run(Engine& E, uint64_t N, uint32_t* minp_host, uint64_t
 uint64_t sophie_germain_count(Engine& E, uint64_t N) {
   uint64_t seeds = (N >= 2) + (N >= 3) + (N >= 5);
   if (N < 11) return seeds;
-  Plan plan;
+  KeptWork work(E);
   uint64_t nw = 0;
-  const uint32_t* wb = sieve_bitmap(E, plan, 0, 2 * N + 2, &nw);
-  DevBuf cnt;
+  const uint32_t* wb = sieve_bitmap(E, work->sieve, 0, 2 * N + 2, &nw);
+  DevBuf& cnt = work->total;
   cnt.reserve(8);
   check_cuda(cudaMemsetAsync(cnt.ptr, 0, 8, E.stream), "memset");
   sophie_germain_kernel<<<E.sm_count * 8, 256, 0, E.stream>>>(wb, N, cnt.as<unsigned long long>());
@@ -565,43 +619,61 @@ uint64_t sophie_germain_count(Engine& E, uint64_t N) {
   return seeds + c;
 }
 
-std::vector<uint64_t> primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count) {
+// Ranges up to this width (72 MB of bitmap) are counted by the run that makes
+// their bitmap, unless they surely hold more than max_count primes; others are
+// counted first, so that an oversized request fails before any bitmap is built.
+constexpr uint64_t kOnePassWidth = 1ull << 31;
+
+PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count) {
+  PrimeList out;
   std::vector<uint64_t> seeds;
   for (uint64_t q : {2ull, 3ull, 5ull}) if (q >= a && q <= b) seeds.push_back(q);
-  if (b < 7) return seeds;
-  // count first, so an oversized request fails before any bitmap is built
+  uint64_t total = seeds.size();
   uint64_t aa = a, bb = b + 1;
-  const uint64_t total = E.run(1, &aa, &bb, nullptr, false)[0].count;
-  if (total > max_count) return std::vector<uint64_t>(max_count + 1, 0);
-  Plan plan;
-  uint64_t nw = 0;
-  const uint32_t* wb = sieve_bitmap(E, plan, a, b + 1, &nw);
-  const uint64_t nblocks = (nw + kExBlockWords - 1) / kExBlockWords;
-  DevBuf bc, bo, outb;
-  bc.reserve(4 * std::max<uint64_t>(nblocks, 1));
-  bo.reserve(8 * std::max<uint64_t>(nblocks, 1));
-  std::vector<uint64_t> res(seeds);
-  if (nblocks) {
-    extract_count_kernel<<<(unsigned)nblocks, kExThreads, 0, E.stream>>>(wb, nw, bc.as<uint32_t>());
-    check_cuda(cudaGetLastError(), "extract_count_kernel");
-    std::vector<uint32_t> counts(nblocks);
-    check_cuda(cudaMemcpyAsync(counts.data(), bc.ptr, 4 * nblocks, cudaMemcpyDeviceToHost, E.stream), "counts");
-    check_cuda(cudaStreamSynchronize(E.stream), "counts");
-    std::vector<uint64_t> offs(nblocks);
-    uint64_t t = 0;
-    for (uint64_t i = 0; i < nblocks; ++i) { offs[i] = t; t += counts[i]; }
-    if (t) {
-      check_cuda(cudaMemcpyAsync(bo.ptr, offs.data(), 8 * nblocks, cudaMemcpyHostToDevice, E.stream), "offsets");
-      outb.reserve(8 * t);
-      extract_write_kernel<<<(unsigned)nblocks, kExThreads, 0, E.stream>>>(
-          wb, nw, plan.host_reqs[0].k_lo, bo.as<uint64_t>(), outb.as<uint64_t>());
-      check_cuda(cudaGetLastError(), "extract_write_kernel");
-      res.resize(seeds.size() + t);
-      check_cuda(cudaMemcpyAsync(res.data() + seeds.size(), outb.ptr, 8 * t, cudaMemcpyDeviceToHost, E.stream), "primes");
-    }
-    check_cuda(cudaStreamSynchronize(E.stream), "in_range");
+  auto listed = [&] {                      // room for `total` primes, or over
+    if (total > max_count) { out.over = true; return false; }
+    if (!total) return false;
+    out.p = static_cast<uint64_t*>(std::malloc(8 * total));
+    if (!out.p) throw std::bad_alloc();
+    std::copy(seeds.begin(), seeds.end(), out.p);
+    out.n = total;
+    return true;
+  };
+  if (b < 7) { listed(); return out; }
+  // the mean density near b, 1 / ln b, less a tenth: below what a range holds
+  if (bb - aa > kOnePassWidth || 0.9 * (double)(bb - aa) / std::log((double)bb) > (double)max_count + 100.0) {
+    total = E.run(1, &aa, &bb, nullptr, false)[0].count;
+    if (total > max_count) { out.over = true; return out; }
   }
-  return res;
+  KeptWork work(E);
+  uint64_t nw = 0;
+  const uint32_t* wb = sieve_bitmap(E, work->sieve, a, b + 1, &nw);
+  const uint64_t nblocks = (nw + kExBlockWords - 1) / kExBlockWords;
+  work->counts.reserve_ahead(4 * std::max<uint64_t>(nblocks, 1));
+  work->offsets.reserve_ahead(8 * std::max<uint64_t>(nblocks, 1));
+  std::vector<uint32_t> counts(nblocks);
+  if (nblocks) {
+    extract_count_kernel<<<(unsigned)nblocks, kExThreads, 0, E.stream>>>(wb, nw, work->counts.as<uint32_t>());
+    check_cuda(cudaGetLastError(), "extract_count_kernel");
+    check_cuda(cudaMemcpyAsync(counts.data(), work->counts.ptr, 4 * nblocks, cudaMemcpyDeviceToHost, E.stream),
+               "counts");
+  }
+  check_cuda(cudaStreamSynchronize(E.stream), "counts");
+  std::vector<uint64_t> offs(nblocks);
+  uint64_t t = 0;
+  for (uint64_t i = 0; i < nblocks; ++i) { offs[i] = t; t += counts[i]; }
+  total = seeds.size() + t;
+  if (!listed() || !t) return out;
+  check_cuda(cudaMemcpyAsync(work->offsets.ptr, offs.data(), 8 * nblocks, cudaMemcpyHostToDevice, E.stream),
+             "offsets");
+  work->primes.reserve_ahead(8 * t);
+  extract_write_kernel<<<(unsigned)nblocks, kExThreads, 0, E.stream>>>(
+      wb, nw, work->sieve.host_reqs[0].k_lo, work->offsets.as<uint64_t>(), work->primes.as<uint64_t>());
+  check_cuda(cudaGetLastError(), "extract_write_kernel");
+  check_cuda(cudaMemcpyAsync(out.p + seeds.size(), work->primes.ptr, 8 * t, cudaMemcpyDeviceToHost, E.stream),
+             "primes");
+  check_cuda(cudaStreamSynchronize(E.stream), "in_range");
+  return out;
 }
 
 }  // namespace vg

@@ -2,6 +2,7 @@
 // check, Sophie Germain count, sorted prime list.  Internal C++.
 #pragma once
 #include <cstdint>
+#include <cstdlib>
 #include <vector>
 
 #include "engine.h"
@@ -37,7 +38,18 @@ uint64_t goldbach_plan_probes(GoldbachPlan* g);
 // Primes p <= N with 2p+1 prime.
 uint64_t sophie_germain_count(Engine& E, uint64_t N);
 
-// Primes q with a <= q <= b, ascending; stops counting at max_count + 1.
-std::vector<uint64_t> primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count);
+// Primes q with a <= q <= b, ascending, in memory from malloc().
+struct PrimeList {
+  uint64_t* p = nullptr;        // null if n == 0 or over
+  uint64_t n = 0;
+  bool over = false;            // more than max_count primes: none are listed
+  PrimeList() = default;
+  PrimeList(PrimeList&& o) noexcept : p(o.p), n(o.n), over(o.over) { o.p = nullptr; }
+  PrimeList(const PrimeList&) = delete;
+  PrimeList& operator=(const PrimeList&) = delete;
+  ~PrimeList() { std::free(p); }
+  uint64_t* take() { uint64_t* r = p; p = nullptr; return r; }
+};
+PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count);
 
 }  // namespace vg

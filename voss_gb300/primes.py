@@ -243,7 +243,7 @@ def _array_result(rc, arr, count) -> list:
     if n == 0:
         return []
     try:
-        return [int(arr[i]) for i in range(n)]
+        return arr[:n]                  # Python ints, converted in one call
     finally:
         _capi._lib.voss_free(arr)
 
