@@ -167,7 +167,7 @@ void Engine::ensure_table(uint64_t pmax) {
       throw Error(VOSS_ERR_INTERNAL, "prime table differs from the kernel's constant table");
   // Plans built earlier keep pointers to the current table: it is retired,
   // not freed, and stays valid for them.
-  for (DevBuf* d : {&dP, &dM, &dR}) {
+  for (DevBuf* d : {&dP, &dM, &dR, &dW, &dWoff}) {
     if (!d->ptr) continue;
     std::unique_ptr<DevBuf> old(new DevBuf());
     old->ptr = d->ptr;
@@ -179,7 +179,14 @@ void Engine::ensure_table(uint64_t pmax) {
   dP.reserve(std::max<size_t>(n, 1) * 4);
   dM.reserve(std::max<size_t>(n, 1) * 8);
   dR.reserve(std::max<size_t>(n, 1) * 8 * 4);
+  std::vector<WheelEntry> W(std::max<size_t>(n, 1));
+  std::vector<uint32_t> Woff(8 * (size_t)wheel_rows((uint32_t)n));
+  build_wheel_table(P.data(), (uint32_t)n, W.data(), Woff.data());
+  dW.reserve(W.size() * sizeof(WheelEntry));
+  dWoff.reserve(Woff.size() * 4);
+  check_cuda(cudaMemcpy(dWoff.ptr, Woff.data(), Woff.size() * 4, cudaMemcpyHostToDevice), "wheel rows");
   if (n) {
+    check_cuda(cudaMemcpy(dW.ptr, W.data(), n * sizeof(WheelEntry), cudaMemcpyHostToDevice), "wheel table");
     check_cuda(cudaMemcpy(dP.ptr, P.data(), n * 4, cudaMemcpyHostToDevice), "table P");
     check_cuda(cudaMemcpy(dM.ptr, M.data(), n * 8, cudaMemcpyHostToDevice), "table M");
     check_cuda(cudaMemcpy(dR.ptr, R.data(), R.size() * 4, cudaMemcpyHostToDevice), "table R");
@@ -199,6 +206,10 @@ uint32_t Engine::primes_below_sq(uint64_t b) const {
 
 uint32_t Engine::index_of(uint32_t p) const {
   return (uint32_t)(std::lower_bound(hP.begin(), hP.end(), p) - hP.begin());
+}
+
+uint32_t Engine::wheel_begin(uint32_t seg_bytes, uint32_t tier_split) const {
+  return wheel_begin_index(seg_bytes, tier_split, [&](uint32_t p) { return index_of(p); });
 }
 
 Config Engine::tuned_for(uint64_t a, uint64_t b, bool batch) const {
@@ -443,7 +454,7 @@ void Plan::load_requests(uint32_t n, const uint64_t* a, const uint64_t* b, uint3
       r.nseg = (r.k_hi - r.k_lo + c.seg_bytes - 1) / c.seg_bytes;
       r.nprimes = E.primes_below_sq(b[i]);
       r.tier_split = E.index_of(c.tier_split);
-      r.tier_huge = E.index_of(c.seg_bytes);
+      r.tier_wheel = E.wheel_begin(c.seg_bytes, r.tier_split);
       smax = std::max(smax, c.seg_bytes);
       // per segment: fill and scan grow with the bytes, setup with the primes
       cost = (double)r.nseg * ((double)c.seg_bytes + 24.0 * r.nprimes);
@@ -559,6 +570,9 @@ void Plan::load_requests(uint32_t n, const uint64_t* a, const uint64_t* b, uint3
   prm.P = E.dP.as<uint32_t>();
   prm.M = E.dM.as<uint64_t>();
   prm.R = E.dR.as<uint32_t>();
+  prm.W = E.dW.as<WheelEntry>();
+  prm.Woff = E.dWoff.as<uint32_t>();
+  prm.ntab = (uint32_t)E.hP.size();
   for (int t = 0; t < kTiles; ++t) {
     prm.tile[t] = E.tile[t].as<uint32_t>();
     prm.tile_stride16[t] = tile_copy_stride(tile_period(t), kMaxSegBytes) / 16;

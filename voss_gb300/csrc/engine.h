@@ -233,6 +233,7 @@ class Engine {
   std::vector<double> hInvPrefix;   // sum of 1/p over table primes [0, i)
   uint64_t table_limit = 0;
   DevBuf dP, dM, dR;            // primes, Barrett constants, class residues (8 per prime)
+  DevBuf dW, dWoff;             // the wheel table (primes by class mod 30) and its row offsets
   // Earlier, smaller copies of the table.  Plans keep pointers to the table
   // they were built with, so a grown table leaves the old one allocated (its
   // primes are a prefix of the new one's) until the engine goes.
@@ -249,6 +250,8 @@ class Engine {
   void ensure_table(uint64_t pmax);
   uint32_t primes_below_sq(uint64_t b) const;   // table primes p with p*p < b
   uint32_t index_of(uint32_t p) const;           // first table index with P >= p
+  // Table index where the wheel tier of segments of seg_bytes starts.
+  uint32_t wheel_begin(uint32_t seg_bytes, uint32_t tier_split) const;
   // Segment size and tier split for one range (offset-regime table, then the
   // built-in rule); batch = tune for the throughput of a batch rather than
   // the latency of this range alone.

@@ -8,8 +8,8 @@
 // serves them: it runs the same sieve and finalize kernels as
 // voss_primes_range_stats, but every byte of device memory it uses beyond
 // the caller's output lives in file-scope static __device__ arrays below
-// (about 29.9 MB per GPU that loads this library, held until the process
-// exits: 24.1 MB of presieve tile copies, 3.6 MB of sieving-prime table and
+// (about 30.6 MB per GPU that loads this library, held until the process
+// exits: 24.1 MB of presieve tile copies, 4.3 MB of sieving-prime table and
 // 2.2 MB of scratch).  It calls no cudaMalloc, cudaFree or allocating library
 // routine.
 //
@@ -72,20 +72,24 @@ struct NaScratch {
   SegRec segs[kNaMaxSegs];
 };
 
-// The scratch of every call (about 2.2 MB), the sieving-prime table (P, M
-// and R: about 3.6 MB) and the presieve tile copies (about 24.1 MB).  In
+// The scratch of every call (about 2.2 MB), the sieving-prime table (P, M,
+// R and W: about 4.3 MB) and the presieve tile copies (about 24.1 MB).  In
 // host code these names are host-side stand-ins; their device addresses
 // come from cudaGetSymbolAddress at set-up.
 static __device__ __align__(256) unsigned char g_na_scratch[sizeof(NaScratch)];
 static __device__ __align__(256) uint32_t g_na_P[kNaStride];
 static __device__ __align__(256) uint64_t g_na_M[kNaStride];
 static __device__ __align__(256) uint32_t g_na_R[8 * kNaStride];
+static __device__ __align__(256) WheelEntry g_na_W[kNaStride];
+static __device__ __align__(256) uint32_t g_na_Woff[8 * wheel_rows(kNaPrimes)];
 static __device__ __align__(256) uint32_t g_na_tiles[kNaTileBytes / 4];
 
 // Host copies of the tables, built once per process in static storage.
 static uint32_t h_P[kNaStride];
 static uint64_t h_M[kNaStride];
 static uint32_t h_R[8 * kNaStride];
+static WheelEntry h_W[kNaStride];
+static uint32_t h_Woff[8 * wheel_rows(kNaPrimes)];
 static uint8_t h_tiles[kNaTileBytes];
 static uint8_t h_tile_base[kMaxTilePeriod];    // one period of a tile
 static uint8_t h_comp[kNaPrimeLimit];
@@ -96,6 +100,8 @@ struct NaDevice {
   NaScratch* scratch = nullptr;
   uint32_t *P = nullptr, *R = nullptr, *tiles = nullptr;
   uint64_t* M = nullptr;
+  WheelEntry* W = nullptr;
+  uint32_t* Woff = nullptr;
   uint32_t sms = 0;
 };
 static NaDevice g_dev[64];
@@ -129,6 +135,7 @@ void build_host_tables() {
     for (int o = 0; o < 8; ++o) h_R[8 * n + o] = (uint32_t)(((p - kW30h[o] % p) % p) * inv30 % p);
     ++n;
   }
+  if (n == kNaPrimes) build_wheel_table(h_P, n, h_W, h_Woff);
   for (int t = 0; t < kTiles; ++t)
     build_tile_copies(kTilePrimes[t], kTilePrimes[t][3] ? 4 : 3, tile_period(t),
                       tile_copy_stride(tile_period(t), kNaSegBytes), h_tile_base, h_tiles + na_tile_offset(t));
@@ -149,11 +156,14 @@ int setup(int dev) {
   if (!h_built) return VOSS_ERR_INTERNAL;
   if (symbol_ptr(&d.scratch, g_na_scratch) != cudaSuccess || symbol_ptr(&d.P, g_na_P) != cudaSuccess ||
       symbol_ptr(&d.M, g_na_M) != cudaSuccess || symbol_ptr(&d.R, g_na_R) != cudaSuccess ||
+      symbol_ptr(&d.W, g_na_W) != cudaSuccess || symbol_ptr(&d.Woff, g_na_Woff) != cudaSuccess ||
       symbol_ptr(&d.tiles, g_na_tiles) != cudaSuccess)
     return VOSS_ERR_CUDA;
   if (cudaMemcpyToSymbol(g_na_P, h_P, sizeof(h_P)) != cudaSuccess ||
       cudaMemcpyToSymbol(g_na_M, h_M, sizeof(h_M)) != cudaSuccess ||
       cudaMemcpyToSymbol(g_na_R, h_R, sizeof(h_R)) != cudaSuccess ||
+      cudaMemcpyToSymbol(g_na_W, h_W, sizeof(h_W)) != cudaSuccess ||
+      cudaMemcpyToSymbol(g_na_Woff, h_Woff, sizeof(h_Woff)) != cudaSuccess ||
       cudaMemcpyToSymbol(g_na_tiles, h_tiles, sizeof(h_tiles)) != cudaSuccess)
     return VOSS_ERR_CUDA;
   int sms = 0;
@@ -243,7 +253,9 @@ extern "C" int voss_primes_range_stats_noalloc(uint64_t a, uint64_t b, voss_rang
     r.nprimes = (uint32_t)(std::upper_bound(h_P, h_P + kNaPrimes, (uint32_t)std::min<uint64_t>(lim, UINT32_MAX)) - h_P);
     const uint32_t split = std::max<uint32_t>(kFirstTablePrime, std::min<uint32_t>(6144, r.seg_bytes / 32));
     r.tier_split = (uint32_t)(std::lower_bound(h_P, h_P + kNaPrimes, split) - h_P);
-    r.tier_huge = (uint32_t)(std::lower_bound(h_P, h_P + kNaPrimes, r.seg_bytes) - h_P);
+    r.tier_wheel = wheel_begin_index(r.seg_bytes, r.tier_split, [](uint32_t p) {
+      return (uint32_t)(std::lower_bound(h_P, h_P + kNaPrimes, p) - h_P);
+    });
   }
   r.bucket_idx = r.nprimes;          // no bucket lists on this path
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -258,6 +270,9 @@ extern "C" int voss_primes_range_stats_noalloc(uint64_t a, uint64_t b, voss_rang
   prm.P = d.P;
   prm.M = d.M;
   prm.R = d.R;
+  prm.W = d.W;
+  prm.Woff = d.Woff;
+  prm.ntab = kNaPrimes;
   for (int t = 0; t < kTiles; ++t) {
     prm.tile[t] = d.tiles + na_tile_offset(t) / 4;
     prm.tile_stride16[t] = tile_copy_stride(tile_period(t), kNaSegBytes) / 16;

@@ -7,16 +7,17 @@
 //      47..59) read at the segment's phase, 16 bytes per load from the tile
 //      copy in which that phase is aligned -- replaces the reference's memset + per-prime
 //      launches for the smallest primes (context.cu:404-414);
-//   2. mark with shared-memory atomicAnd, in work units handed out heaviest
-//      first by a shared counter: primes 61 <= p < split one warp each
-//      (lane = residue class x stream, fixed bit mask per stream); split <=
-//      p < S four per warp-round (lane = prime x class); p >= S two per
-//      lane (at most one hit per class); primes from the request's bucket
-//      split on come from the segment's bucket list, 1024 entries per unit,
-//      read coalesced from HBM (filled by bucket_fill_kernel).  Each stream
-//      starts at max(p^2, segment low), as the reference's
-//      sieve_w30_seg_kernel does (sieve.cu:10-37, start offsets
-//      context.cu:354-388);
+//   2. mark with shared-memory atomicAnd, in work units handed out by a
+//      shared counter: primes 61 <= p < split one warp each (lane = residue
+//      class x stream, fixed bit mask per stream); split <= p < S/16 four per
+//      warp-round (lane = prime x class); from S/16 on a lane per prime, 32
+//      primes of one class mod 30 at a time (the wheel tier); primes from the
+//      request's bucket split on come from the segment's bucket list, 1024
+//      entries per unit, read coalesced from HBM (filled by
+//      bucket_fill_kernel).  The reference's sieve_w30_seg_kernel starts each
+//      stream at p^2 (sieve.cu:10-37, start offsets context.cu:354-388); here
+//      they start at the segment, and a low segment's own sieving primes are
+//      set again;
 //   3. reduce in the same CTA: popcount (count), masked popcount (p mod 4,
 //      p mod 3), and an ordered gap scan with a warp max-scan carrying the
 //      previous prime, histogram in shared memory -- replaces extract +
@@ -41,6 +42,7 @@ __device__ __forceinline__ uint32_t w30(uint32_t o) {
 }
 
 __constant__ ConstPrimeTable cTab = make_const_prime_table();
+__constant__ WheelClasses cWheel = make_wheel_classes();
 
 // x mod p by Barrett reduction with m = floor((2^64-1)/p).
 __device__ __forceinline__ uint32_t mod_barrett(uint64_t x, uint32_t p, uint64_t m) {
@@ -62,11 +64,54 @@ __device__ __forceinline__ uint32_t lift_to_square(uint32_t s, uint64_t k0, uint
   return s2 < nbytes ? (uint32_t)s2 : nbytes;
 }
 
-// Clear the candidate of byte j, class o, given keep = ~(1 << o): the mask
-// is keep rotated to byte j & 3 of its word (a funnel shift uses its count
-// mod 32, so 8 * j rotates by 8 * (j & 3)).
-__device__ __forceinline__ void clear_bit(uint32_t* seg, uint32_t j, uint32_t keep) {
-  atomicAnd(seg + (j >> 2), __funnelshift_l(keep, keep, j << 3));
+// A value that is the same in every lane, as a warp-uniform register: the
+// compiler then branches on it without divergence bookkeeping (a quarter of the
+// marking's instructions went there when units and bounds were read by shuffle
+// or from shared memory).
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __reduce_max_sync(0xFFFFFFFFu, x); }
+
+// Clear the candidate at shared address j (the segment's start plus its byte;
+// the start is a multiple of four), given keep = ~(1 << class): the mask is keep
+// with its low byte moved to byte j & 3 of the word, which a byte permute in
+// backward-extract mode does from j itself (it reads two selector bits).
+__device__ __forceinline__ void clear_at(uint32_t j, uint32_t keep) {
+  asm volatile(
+      "{\n\t.reg .b32 m, a;\n\t"
+      "prmt.b32.b4e m, %1, %1, %0;\n\t"
+      "and.b32 a, %0, -4;\n\t"
+      "red.shared.and.b32 [a], m;\n\t}"
+      :: "r"(j), "r"(keep) : "memory");
+}
+
+// The same where j < end, as one predicated instruction: a branch around it
+// costs more issue slots than the address and mask that idle lanes compute.
+__device__ __forceinline__ void clear_below(uint32_t j, uint32_t keep, uint32_t end) {
+  asm volatile(
+      "{\n\t.reg .b32 m, a;\n\t.reg .pred p;\n\t"
+      "setp.lt.u32 p, %0, %2;\n\t"
+      "prmt.b32.b4e m, %1, %1, %0;\n\t"
+      "and.b32 a, %0, -4;\n\t"
+      "@p red.shared.and.b32 [a], m;\n\t}"
+      :: "r"(j), "r"(keep), "r"(end) : "memory");
+}
+
+// A word at shared address a with a mask at hand, always or where on.
+__device__ __forceinline__ void and_word(uint32_t a, uint32_t mask) {
+  asm volatile("red.shared.and.b32 [%0], %1;" :: "r"(a), "r"(mask) : "memory");
+}
+__device__ __forceinline__ void and_word_if(uint32_t a, uint32_t mask, bool on) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p red.shared.and.b32 [%0], %1;\n\t}"
+               :: "r"(a), "r"(mask), "r"((uint32_t)on) : "memory");
+}
+
+// The same for a candidate given as bit index v = 8 * byte + class of the
+// segment at shared address seg: its word is v / 32 and its mask 0xFFFFFFFE
+// rotated by v (a funnel shift takes its count mod 32).
+__device__ __forceinline__ void clear_bit(uint32_t seg, uint32_t v) {
+  and_word(seg + 4u * (v >> 5), __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, v));
+}
+__device__ __forceinline__ void clear_bit_below(uint32_t seg, uint32_t v, uint32_t end) {
+  if (v < end) clear_bit(seg, v);
 }
 
 // The eight class residues of table prime i (32 bytes, two vector loads).
@@ -116,7 +161,7 @@ __device__ __forceinline__ void record_gap(const GapSink& sk, uint32_t vprev, ui
 // live in wheel byte 0, 31 in byte 1), 1, and the request's ends.
 struct SegItem {
   uint64_t item, k0, bbase;
-  uint32_t req, nbytes, np, split, huge, rflags, bcnt, valid;
+  uint32_t req, nbytes, np, split, wheel, rflags, bcnt, valid;
   uint32_t and0, or0, keep0, keepl;
 };
 
@@ -176,7 +221,7 @@ __device__ __noinline__ void claim_item(unsigned long long* queue, const ReqDesc
     }
     d.item = item; d.valid = 1;
     d.req = r; d.k0 = k0; d.nbytes = nb; d.np = a;
-    d.split = R.tier_split; d.huge = R.tier_huge; d.rflags = R.rflags;
+    d.split = R.tier_split; d.wheel = R.tier_wheel; d.rflags = R.rflags;
     uint32_t and0 = ~0u, or0 = 0u, keep0 = ~0u, keepl = ~0u;
     if (k0 == 0) and0 = ~1u;                               // 1 is not prime
     if (k0 < 3) or0 = (uint32_t)(kTilePrimeBits >> (8u * k0));   // the tile primes are
@@ -209,6 +254,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
 sieve_segments_kernel(const SieveParams prm) {
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* seg = smem;
+  const uint32_t sseg = (uint32_t)__cvta_generic_to_shared(seg);
   uint32_t* shist = seg + (prm.seg_bytes >> 2);
   WarpRec* wrec = reinterpret_cast<WarpRec*>(shist + kSmemHistCopies * kSmemStride);
   uint4* btab = reinterpret_cast<uint4*>(wrec + kMaxThreads / 32);   // the gap scan's byte table
@@ -289,42 +335,64 @@ sieve_segments_kernel(const SieveParams prm) {
     }
     __syncthreads();
 
-    // 2. marking.  Work units, heaviest first, handed out by a shared counter:
+    // 2. marking.  Work units handed out by a shared counter:
     //    units [0, nsmall): one prime each, p < split: a warp per prime, lane
     //      = (class o, stream h of 4); a stream steps 4p bytes = p words, so
     //      its bit mask never changes;
-    //    then 32 primes each, split <= p < S: lanes = (prime q of 4, class
+    //    then 32 primes each up to the wheel tier: lanes = (prime q of 4, class
     //      o), eight rounds of four primes, loads of all rounds issued before
     //      any marking so their latency overlaps;
-    //    then 64 primes each, p >= S (two per lane), then the bucket units.
+    //    then 64 primes of one class mod 30 each (the wheel tier, two per
+    //      lane), then kBucketUnit entries of the segment's bucket list each.
     {
-      // unit layout: [0, nsmall) small primes, then 32-prime units of the mid
-      // tier (split <= p < S), then 64-prime units of the huge tier (p >= S),
-      // then kBucketUnit-entry units of the segment's bucket list
-      const uint32_t nsmall = S.split < np ? S.split : np;
-      const uint32_t hbeg = S.huge < np ? max(S.huge, nsmall) : np;
-      const uint32_t nmidu = (hbeg - nsmall + 31u) / 32u;
-      const uint32_t nhugeu = (np - hbeg + 2u * kHugeHalf - 1u) / (2u * kHugeHalf);
-      const uint32_t nscan = nsmall + nmidu + nhugeu;
-      const uint32_t bcnt = S.bcnt;
+      const uint32_t unp = uniform(np), unb = uniform(nbytes);
+      const uint32_t wheel = uniform(S.wheel);
+      const uint32_t nsmall = min(uniform(S.split), unp);
+      const uint32_t mend = wheel < unp ? max(wheel, nsmall) : unp;
+      const uint32_t nmidu = (mend - nsmall + 31u) / 32u;
+      // the wheel tier's run of each class (lane = class): positions wbeg ..
+      // wend - 1 of the wheel table, and the units of classes 0 .. lane.  The
+      // end is rounded up to a row: the primes past np that this adds clear
+      // composites only (and themselves, see the restoring below).
+      uint32_t wbeg = 0, wend = 0;
+      if (lane < 8u && wheel < unp) {
+        wbeg = __ldg(prm.Woff + 8u * (wheel / kWheelRow) + lane);
+        wend = __ldg(prm.Woff + 8u * ((unp + kWheelRow - 1u) / kWheelRow) + lane);
+      }
+      // primes per unit, 2^wlog: claiming a unit costs about as much as
+      // marking 32 primes, but every warp should get several units
+      uint32_t wlog = 5;
+      while (wlog < kWheelUnitLog2Max && mend + (256u << wlog) <= unp) ++wlog;
+      uint32_t wincl = (wend - wbeg + (1u << wlog) - 1u) >> wlog;
+#pragma unroll
+      for (int d = 1; d < 8; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, wincl, d);
+        if ((int)lane >= d) wincl += t;
+      }
+      const uint32_t nscan = nsmall + nmidu + uniform(lane == 7u ? wincl : 0u);
+      // x mod p for the wheel tier (p > 2^10): q = hi32((x >> 10) * floor(2^42
+      // / p)) is x / p or up to 2 less, so 32 bits of remainder suffice
+      const uint32_t k0s = uniform((uint32_t)(k0 >> 10)), k0l = uniform((uint32_t)k0);
+      const uint32_t bcnt = uniform(S.bcnt);
       const uint64_t bbase = S.bbase;
       if (warp == 0)                                // overlaps the marking
         claim_item(prm.queue, prm.reqs, prm.P, prm.bcount, prm.item_lo, item_end, prm.list_seg0, nreq,
                    s_item[cur ^ 1u], lane);
       const uint32_t nunits = nscan + (bcnt + kBucketUnit - 1) / kBucketUnit;
       const uint32_t o = lane & 7u, h = lane >> 3;
+      const uint32_t send = sseg + unb;             // shared address past the segment's end
       for (;;) {
         uint32_t u = 0;
         if (lane == 0) u = atomicAdd(&s_ctr, 1u);
-        u = __shfl_sync(0xFFFFFFFFu, u, 0);
+        u = uniform(u);
         if (u >= nunits) break;
         if (u < nsmall) {
           const bool cst = u < kConstPrimes;
           const uint32_t p = cst ? cTab.p[u] : __ldg(prm.P + u);
           const uint32_t m = mod_barrett(k0, p, cst ? (uint64_t)cTab.m[u] : __ldg(prm.M + u));
           const uint32_t r = __ldg(prm.R + 8u * u + o);
-          uint32_t s = r >= m ? r - m : r + p - m;
-          if (30ull * k0 < (uint64_t)p * p) s = lift_to_square(s, k0, p, o, nbytes);
+          uint32_t s = r - m;
+          s = min(s, s + p);
           // This lane's stream: bytes j0 + 4 p i = words w0 + p i with one
           // mask, n of them in the segment.  All 32 streams step p words, so
           // their banks shift alike: a lane that starts at the step rot
@@ -337,7 +405,7 @@ sieve_segments_kernel(const SieveParams prm) {
           const uint32_t j0 = s + h * p;
           const uint32_t c = j0 & 3u;
           const uint32_t mask = ~(1u << ((c << 3) | o));
-          const uint32_t lim = (nbytes - c + 3u) >> 2;      // word w holds byte 4w + c < nbytes
+          const uint32_t lim = (unb - c + 3u) >> 2;         // word w holds byte 4w + c < nbytes
           const uint32_t w0 = j0 >> 2;
           const uint32_t n = w0 < lim ? (lim - w0 + p - 1u) / p : 0u;
           const uint32_t pinv = p * (2u - p * p);           // p^-1 mod 64 (p odd, p*p = 1 mod 8)
@@ -345,14 +413,21 @@ sieve_segments_kernel(const SieveParams prm) {
           if (rot >= n) rot = n ? rot % n : 0u;
           const uint32_t first = n - rot;                    // steps before the wrap
           const uint32_t k1 = __reduce_min_sync(0xFFFFFFFFu, first);
-          const uint32_t kmax = __reduce_max_sync(0xFFFFFFFFu, n);
-          uint32_t* q = seg + w0 + p * rot;
+          const uint32_t k2 = __reduce_min_sync(0xFFFFFFFFu, n);
+          const uint32_t k3 = __reduce_max_sync(0xFFFFFFFFu, n);
+          const uint32_t p4 = 4u * p, turn = n * p4;
+          uint32_t q = sseg + 4u * w0 + p4 * rot;
           uint32_t k = 0;
+#pragma unroll 16
+          for (; k < k1; ++k, q += p4) and_word(q, mask);
 #pragma unroll 8
-          for (; k < k1; ++k, q += p) atomicAnd(q, mask);
-          for (; k < kmax; ++k, q += p) {
-            if (k == first) q -= n * p;                      // wrap to step 0
-            if (k < n) atomicAnd(q, mask);
+          for (; k < k2; ++k, q += p4) {                     // some lanes have wrapped
+            if (k == first) q -= turn;
+            and_word(q, mask);
+          }
+          for (; k < k3; ++k, q += p4) {                     // some lanes are done
+            if (k == first) q -= turn;
+            and_word_if(q, mask, k < n);
           }
         } else if (u >= nscan) {
           // bucket list of this segment: primes >= the bucket split whose
@@ -367,73 +442,154 @@ sieve_segments_kernel(const SieveParams prm) {
             atomicAnd(seg + (v >> 5), __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, v));
           }
         } else if (u >= nsmall + nmidu) {
-          // huge tier: p >= S, at most one hit per class; 64-prime units, a
-          // lane per prime in each of two halves whose table loads are all
-          // issued first; the eight classes unrolled, clears predicated.
-          const uint32_t ib = hbeg + 2u * kHugeHalf * (u - nsmall - nmidu) + lane;
-          uint32_t pq[2], rq[2][8];
-          uint64_t mq[2];
+          // wheel tier: a lane per prime of one class mod 30, its eight hits
+          // per turn of p bytes in the order of their cofactors w mod 30: the
+          // first lies at t w + const - k0 (mod p), the next ones follow by p.
+          // With the eight residues of each prime read from memory (44 bytes
+          // where this takes 8, as many shared-memory wavefronts as the
+          // clears), a 64-bit reduction and a branch per clear, the primes
+          // above the segment took 168 instructions per prime and segment and
+          // those below it 13 per clear; now about 100 (60 from 2.5 segments
+          // on) and 6.  [9*10^11, 10^12): 20.8 -> 16.5 ms with the uniform
+          // unit bounds.  What bounds it: shared-memory wavefronts (3.5 per
+          // atomic on random banks) below the segment size, issue above.
+          const uint32_t wu = u - nsmall - nmidu;
+          const uint32_t cls = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, lane < 8u && wu >= wincl));
+          const uint32_t ubeg = __shfl_sync(0xFFFFFFFFu, wincl, (cls + 31u) & 31u);
+          const uint32_t cend = __shfl_sync(0xFFFFFFFFu, wend, cls);
+          uint32_t i = __shfl_sync(0xFFFFFFFFu, wbeg, cls) + ((wu - (cls ? ubeg : 0u)) << wlog) + lane;
+          const uint32_t cc = w30(cls);
+          const WheelClass& C = cWheel.c[cls];
+          const uint2* __restrict__ W = reinterpret_cast<const uint2*>(prm.W);
+          // past the class's end a lane repeats its last prime: the same
+          // clears again
+          uint2 e = __ldg(W + min(i, cend - 1u));
+          const uint32_t pfirst = __reduce_min_sync(0xFFFFFFFFu, 30u * e.x + cc);
+          uint32_t left = 1u << (wlog - 5u);            // batches of 32 primes
+          if (pfirst >= unb) {
+            // at most one hit per class: positions as bit indices 8 * byte +
+            // class, whose low bits also give the mask
+            uint32_t step[8];
 #pragma unroll
-          for (uint32_t q = 0; q < 2; ++q) {
-            // past the table end a lane repeats the last prime: its clears
-            // are the same bits again
-            const uint32_t i = min(ib + kHugeHalf * q, np - 1u);
-            pq[q] = __ldg(prm.P + i);
-            mq[q] = __ldg(prm.M + i);
-            load_residues(prm.R, i, rq[q]);
-          }
+            for (int j = 0; j < 8; ++j) step[j] = C.bstep[j];
+            // from 2.5 segments on, cofactors w_j and w_(j+4) lie 12/30 to
+            // 18/30 of p apart, so at most one of the two hits is inside
+            const bool sparse = 2u * pfirst >= 5u * unb;
+            const uint32_t end = 8u * unb;
+            for (;;) {
+              const uint32_t p = 30u * e.x + cc;
+              uint32_t m = k0l - __umulhi(k0s, e.y) * p;
+              const uint32_t t2 = 16u * e.x, t4 = 32u * e.x, t6 = 48u * e.x, p8 = 8u * p;
+              uint32_t y = 8u * e.x + step[0];
+              if (--left) e = __ldg(W + min(i += 32u, cend - 1u));
+              m = min(m, m - p);
+              m = min(m, m - p);
+              y -= 8u * m;
+              uint32_t v[8];
+              v[0] = min(y, y + p8);
 #pragma unroll
-          for (uint32_t q = 0; q < 2; ++q) {
-            const uint32_t p = pq[q];
-            const uint32_t m = mod_barrett(k0, p, mq[q]);
-            const uint64_t p2 = (uint64_t)p * p;
-            const bool low = 30ull * k0 < p2;
-            uint32_t sv[8];
+              for (int j = 1; j < 8; ++j) {
+                // W30 steps 6 4 2 4 2 4 6
+                y += (j == 1 || j == 7 ? t6 : j == 3 || j == 5 ? t2 : t4) + step[j];
+                v[j] = min(y, y + p8);
+              }
+              if (sparse) {
 #pragma unroll
-            for (uint32_t t = 0; t < 8; ++t) sv[t] = rq[q][t] >= m ? rq[q][t] - m : rq[q][t] + p - m;
-            // p >= the segment: sv[t] is the class's only candidate here, so
-            // below p*p there is none (the next one is sv[t] + p).  The test
-            // sits apart from the clears, under one branch taken by few
-            // segments.
-            if (low) {
+                for (int j = 0; j < 4; ++j) clear_bit_below(sseg, min(v[j], v[j + 4]), end);
+              } else {
 #pragma unroll
-              for (uint32_t t = 0; t < 8; ++t)
-                if (30ull * (k0 + sv[t]) + w30(t) < p2) sv[t] = nbytes;
+                for (int j = 0; j < 8; ++j) clear_bit_below(sseg, v[j], end);
+              }
+              if (!left) break;
             }
+          } else {
+            // several hits per class; whole turns of the batch's largest
+            // prime need no test
+            uint32_t step[8], keep[8];
 #pragma unroll
-            for (uint32_t t = 0; t < 8; ++t)
-              if (sv[t] < nbytes) clear_bit(seg, sv[t], ~(1u << t));
+            for (int j = 0; j < 8; ++j) { step[j] = C.step[j]; keep[j] = C.keep[j]; }
+            for (;;) {
+              const uint32_t p = 30u * e.x + cc;
+              uint32_t m = k0l - __umulhi(k0s, e.y) * p;
+              m = min(m, m - p);
+              m = min(m, m - p);
+              const uint32_t t2 = 2u * e.x, t4 = 4u * e.x, t6 = 6u * e.x;
+              uint32_t pos[8];
+              uint32_t y = e.x - m;                     // offset of the hit of w = 1, mod p
+              pos[0] = min(y, y + p);
+#pragma unroll
+              for (int j = 1; j < 8; ++j) {
+                y += (j == 1 || j == 7 ? t6 : j == 3 || j == 5 ? t2 : t4) + step[j];
+                pos[j] = min(y, y + p);
+              }
+              uint32_t n = __umulhi(unb, e.y) >> 10;
+              if ((n + 1u) * p <= unb) ++n;             // floor(nbytes / p)
+              if (--left) e = __ldg(W + min(i += 32u, cend - 1u));
+#pragma unroll
+              for (int j = 0; j < 8; ++j) pos[j] += sseg;
+              const uint32_t nall = __reduce_min_sync(0xFFFFFFFFu, n);
+              const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, n) + 1u;
+              uint32_t k = 0;
+#pragma unroll 1
+              for (; k < nall; ++k) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) { clear_at(pos[j], keep[j]); pos[j] += p; }
+              }
+#pragma unroll 1
+              for (; k < nmax; ++k) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) { clear_below(pos[j], keep[j], send); pos[j] += p; }
+              }
+              if (!left) break;
+            }
           }
         } else {
-          // mid tier: p and k0 mod p once per prime (lane = prime), then
-          // shuffled to the (prime, class) lanes of each round.
+          // mid tier: p, k0 mod p and the whole turns of p once per prime (lane
+          // = prime), then shuffled to the (prime, class) lanes of each round.
+          // Past the tier's end a lane repeats its last prime.
           const uint32_t base = nsmall + 32u * (u - nsmall);
-          const uint32_t im = base + lane;
-          const bool okm = im < hbeg;
-          const uint32_t pm = okm ? __ldg(prm.P + im) : 0u;
-          const uint32_t mm = okm ? mod_barrett(k0, pm, __ldg(prm.M + im)) : 0u;
-          const bool low_any = __any_sync(0xFFFFFFFFu, okm && 30ull * k0 < (uint64_t)pm * pm);
+          const uint32_t im = min(base + lane, mend - 1u);
+          const uint32_t pm = __ldg(prm.P + im);
+          const uint32_t mm = mod_barrett(k0, pm, __ldg(prm.M + im));
+          const uint32_t nm = unb / pm;
           const uint32_t keep = ~(1u << o);
           uint32_t rr[8];
 #pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const uint32_t i = base + 4u * t + h;
-            rr[t] = i < hbeg ? __ldg(prm.R + 8u * i + o) : 0u;
-          }
+          for (int t = 0; t < 8; ++t) rr[t] = __ldg(prm.R + 8u * min(base + 4u * t + h, mend - 1u) + o);
 #pragma unroll
           for (int t = 0; t < 8; ++t) {
             const uint32_t p = __shfl_sync(0xFFFFFFFFu, pm, 4 * t + h);
             const uint32_t m = __shfl_sync(0xFFFFFFFFu, mm, 4 * t + h);
-            if (!p) continue;
-            uint32_t s = rr[t] >= m ? rr[t] - m : rr[t] + p - m;
-            if (low_any && 30ull * k0 < (uint64_t)p * p) s = lift_to_square(s, k0, p, o, nbytes);
+            uint32_t s = rr[t] - m;
+            s = min(s, s + p);
+              const bool mine = (lane >> 2) == (uint32_t)t;
+            const uint32_t nall = __reduce_min_sync(0xFFFFFFFFu, mine ? nm : ~0u);
+            const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, mine ? nm : 0u) + 1u;
+            uint32_t j = sseg + s, k = 0;
 #pragma unroll 8
-            for (uint32_t j = s; j < nbytes; j += p) clear_bit(seg, j, keep);
+            for (; k < nall; ++k, j += p) clear_at(j, keep);
+#pragma unroll 2
+            for (; k < nmax; ++k, j += p) clear_below(j, keep, send);
           }
         }
       }
     }
     __syncthreads();
+    // Multiples of p below p*p are cleared too; they are composite anyway, but
+    // for p itself.  Only a segment that starts below 128 bytes can hold a
+    // prime that sieves it (p*p < 30 (k0 + nbytes) and p >= 30 k0 need k0 <=
+    // 86; the rounding to a row adds primes of less than 3840): there they are
+    // set again.  This spares every hit a p*p test.
+    if (k0 < 128u) {
+      const uint32_t nset = min((np + kWheelRow - 1u) / kWheelRow * kWheelRow, prm.ntab);
+      for (uint32_t i = tid; i < nset; i += nthr) {
+        const uint32_t p = __ldg(prm.P + i), k = p / 30u;
+        if (k < k0 || k - (uint32_t)k0 >= nbytes) continue;
+        const uint32_t v = 8u * (k - (uint32_t)k0) + (p % 30u) * 4u / 15u;    // W30[o] * 4 / 15 = o
+        atomicOr(seg + (v >> 5), 1u << (v & 31u));
+      }
+      __syncthreads();
+    }
     if (tid == 0) s_ctr = 0;                        // every unit is taken: reset for the next segment
 
     // 3. reductions: each thread scans one contiguous run of words (odd

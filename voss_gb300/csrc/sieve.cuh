@@ -98,6 +98,79 @@ constexpr ConstPrimeTable make_const_prime_table() {
   return t;
 }
 
+// The wheel table: the table primes p = 30 t + c again, grouped by their class
+// c mod 30 (classes in W30 order, ascending within a class), as {t, inv} with
+// inv = floor(2^42 / p).  For one class everything but t is fixed: the
+// multiple p (30 a + w) lies in wheel byte p a + t w + floor(c w / 30), on the
+// bit of residue c w mod 30.  So a lane needs 8 bytes of table per prime, not
+// the eight residues.  Row r of the offsets gives, per class, the table
+// position of its first prime with table index >= kWheelRow r.
+constexpr uint32_t kWheelRow = 64;
+// The tier's primes must exceed 2^10 (inv < 2^32, see the kernel; its wheel bytes
+// k0 stay below 2^42).  From 3000 on a class has enough primes of one size for
+// its batches of 32 (a 10^7 range: 51 us from 1031 on, 49 us from 3001).
+constexpr uint32_t kWheelMinPrime = 3001;
+struct WheelEntry { uint32_t t, inv; };
+struct WheelClass {
+  // with o_j the bit of residue c w_j mod 30:
+  uint32_t step[8];         // floor(c w_j / 30) - floor(c w_(j-1) / 30) (step[0] = 0)
+  uint32_t keep[8];         // ~(1 << o_j)
+  uint32_t bstep[8];        // the same steps in bit indices: 8 step[j] + o_j - o_(j-1) (bstep[0] = o_0)
+};
+struct WheelClasses { WheelClass c[8]; };
+constexpr WheelClasses make_wheel_classes() {
+  WheelClasses r{};
+  for (uint32_t k = 0; k < 8; ++k) {
+    const uint32_t c = (uint32_t)((kW30Packed >> (8 * k)) & 0xFFu);
+    uint32_t prev = 0, prevo = 0;
+    for (uint32_t j = 0; j < 8; ++j) {
+      const uint32_t w = (uint32_t)((kW30Packed >> (8 * j)) & 0xFFu);
+      const uint32_t q = c * w / 30u, res = c * w % 30u;
+      uint32_t oj = 0;
+      for (uint32_t o = 0; o < 8; ++o)
+        if (((kW30Packed >> (8 * o)) & 0xFFu) == res) oj = o;
+      r.c[k].step[j] = q - prev;
+      r.c[k].keep[j] = ~(1u << oj);
+      r.c[k].bstep[j] = 8u * (q - prev) + oj - prevo;
+      prev = q;
+      prevo = oj;
+    }
+  }
+  return r;
+}
+__host__ __device__ constexpr uint32_t wheel_rows(uint32_t nprimes) { return nprimes / kWheelRow + 2u; }
+// Host: the wheel table of the ascending table primes P[0..n): W gets n
+// entries, off 8 * wheel_rows(n).
+inline void build_wheel_table(const uint32_t* P, uint32_t n, WheelEntry* W, uint32_t* off) {
+  uint32_t cls[30] = {};
+  for (uint32_t k = 0; k < 8; ++k) cls[(kW30Packed >> (8 * k)) & 0xFFu] = k;
+  uint32_t at[8] = {};
+  for (uint32_t i = 0; i < n; ++i)
+    for (uint32_t k = cls[P[i] % 30u] + 1; k < 8; ++k) ++at[k];      // classes start after the smaller ones
+  for (uint32_t r = 0; r < wheel_rows(n); ++r) {
+    for (uint32_t k = 0; k < 8; ++k) off[8 * r + k] = at[k];
+    for (uint32_t i = kWheelRow * r; i < n && i < kWheelRow * (r + 1); ++i) {
+      WheelEntry& e = W[at[cls[P[i] % 30u]]++];
+      e.t = P[i] / 30u;
+      e.inv = P[i] > 1024u ? (uint32_t)((1ull << 42) / P[i]) : 0u;
+    }
+  }
+}
+
+// Where the wheel tier of segments of seg_bytes starts: the first row of table
+// primes from seg_bytes / kWheelDiv on, not below the warp-per-prime tier
+// (index split) nor kWheelMinPrime.  index_of(p): first table index >= p.
+// Further down a batch of 32 primes of one class spans too wide a range of p:
+// its last turns run half idle ([0, 10^10) 1.313 / 1.319 / 1.335 ms, [9*10^11,
+// 10^12) 17.0 / 16.8 / 16.8 ms with the tier from S/8 / S/16 / S/32 on).
+constexpr uint32_t kWheelDiv = 16;
+template <class IndexOf>
+inline uint32_t wheel_begin_index(uint32_t seg_bytes, uint32_t split, IndexOf index_of) {
+  const uint32_t from = seg_bytes / kWheelDiv > kWheelMinPrime ? seg_bytes / kWheelDiv : kWheelMinPrime;
+  const uint32_t i = index_of(from) > split ? index_of(from) : split;
+  return (i + kWheelRow - 1u) / kWheelRow * kWheelRow;
+}
+
 // The presieve tiles are stored as kTileShifts copies, copy c starting c
 // bytes into the periodic pattern, so that the pattern at any byte phase
 // starts on a 16-byte boundary of one copy: the fill reads them with
@@ -149,7 +222,7 @@ struct ReqDesc {
   uint32_t nprimes;         // table primes p (>= 61) with p*p < b
   uint32_t seg_bytes;       // this request's segment size (<= the launch's)
   uint32_t tier_split;      // table index of the first mid-tier prime
-  uint32_t tier_huge;       // table index of the first prime >= seg_bytes
+  uint32_t tier_wheel;      // table index of the first wheel-tier prime (a multiple of kWheelRow)
   uint32_t rflags;          // kReqGaps: gap histogram and largest gap wanted
   uint32_t bucket_idx;      // table index of the first bucket prime (= nprimes: none)
   uint64_t bucket_base;     // first entry of this request's bucket lists
@@ -163,7 +236,7 @@ constexpr uint32_t kReqGaps = 1u;
 // reusing the same memory (fill-kernel shared counts, 16-bit packing, and
 // window offsets below 2^30 bytes).
 constexpr uint32_t kMaxBucketSegs = 4096;
-constexpr uint32_t kHugeHalf = 32;           // primes per half of a huge-tier work unit (one per lane)
+constexpr uint32_t kWheelUnitLog2Max = 8;    // wheel-tier primes per work unit: 2^5 .. 2^8
 constexpr uint32_t kBucketUnit = 1024;       // list entries per work unit of the sieve kernel
 constexpr uint32_t kFillPrimes = 256;        // bucket primes per fill work item
 constexpr uint32_t kFillHits = 16384;        // list entries per fill work item, about
@@ -247,6 +320,9 @@ struct SieveParams {
   const uint32_t* P;         // table primes >= 61, ascending
   const uint64_t* M;         // floor((2^64-1)/p), for x mod p
   const uint32_t* R;         // R[8 * i + o]: k = R (mod p) <=> p | 30k+W30[o] (32 B per prime)
+  const WheelEntry* W;       // the wheel table and its row offsets
+  const uint32_t* Woff;
+  uint32_t ntab;             // table primes
   const uint32_t* tile[kTiles];      // presieve tiles: kTileShifts shifted copies each
   uint32_t tile_stride16[kTiles];    // 16-byte units per copy
   uint32_t seg_bytes;        // the largest segment of the launch (shared memory)
