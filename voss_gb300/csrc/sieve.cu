@@ -140,8 +140,8 @@ __device__ __forceinline__ void record_gap(const GapSink& sk, uint32_t vprev, ui
   const uint32_t g = v - vprev;
   const uint32_t bin = g >> 1;
   atomicAdd(sk.shist + min(bin, (uint32_t)kSmemBins), 1u);
-  // rare: a new maximum, g >= kLargeGap, or g >= 2*kSmemBins (> kLargeGap)
-  if (g > min(maxg, kLargeGap - 1u)) {
+  // rare: a new maximum or g >= 2 * kSmemBins (which covers g >= kLargeGap)
+  if (g > min(maxg, 2u * (uint32_t)kSmemBins - 1u)) {
     if (g > maxg) { maxg = g; maxgs = vprev; }
     if (bin >= (uint32_t)kSmemBins)
       atomicAdd(&sk.acc->hist[bin < (uint32_t)kHistBins ? bin : kHistBins - 1], 1ull);
@@ -153,6 +153,44 @@ __device__ __forceinline__ void record_gap(const GapSink& sk, uint32_t vprev, ui
       }
     }
   }
+}
+
+static_assert(2u * (uint32_t)kSmemBins <= kLargeGap, "gaps from kLargeGap on must leave the shared bins");
+
+// Value of bit b of a word, relative to the word's first integer.
+__device__ __forceinline__ uint32_t word_value(uint32_t b) { return 30u * (b >> 3) + w30(b & 7u); }
+
+// A thread's run of words, prime by prime: its largest gap (the earliest on
+// ties), and the gaps beyond the shared bins.
+__device__ __noinline__ uint2 walk_run(GapSink sk, const uint32_t* seg, uint32_t wbeg, uint32_t wend) {
+  uint32_t best = 0, at = 0, pv = 0;
+  bool any = false;
+  for (uint32_t wi = wbeg; wi < wend; ++wi) {
+    for (uint32_t w = seg[wi]; w; w &= w - 1u) {
+      const uint32_t v = 120u * wi + word_value(__ffs(w) - 1u);
+      const uint32_t g = v - pv;
+      if (any && g > best) { best = g; at = pv; }
+      if (any && g >= 2u * (uint32_t)kSmemBins) {
+        const uint32_t bin = g >> 1;
+        atomicAdd(&sk.acc->hist[bin < (uint32_t)kHistBins ? bin : kHistBins - 1], 1ull);
+        if (g >= kLargeGap) {
+          const unsigned idx = atomicAdd(sk.n_large, 1u);
+          if (idx < sk.cap) {
+            LargeGapRec r; r.pos = sk.base + v; r.gap = g; r.req = sk.req;
+            sk.large[idx] = r;
+          }
+        }
+      }
+      pv = v;
+      any = true;
+    }
+  }
+  return make_uint2(best, at);
+}
+
+// Add one to the 32-bit counter at shared address a.
+__device__ __forceinline__ void count_one(uint32_t a) {
+  asm volatile("red.shared.add.u32 [%0], 1;" :: "r"(a) : "memory");
 }
 
 // A claimed (request, segment) work item with what the CTA needs of it.
@@ -257,26 +295,61 @@ sieve_segments_kernel(const SieveParams prm) {
   const uint32_t sseg = (uint32_t)__cvta_generic_to_shared(seg);
   uint32_t* shist = seg + (prm.seg_bytes >> 2);
   WarpRec* wrec = reinterpret_cast<WarpRec*>(shist + kSmemHistCopies * kSmemStride);
-  uint4* btab = reinterpret_cast<uint4*>(wrec + kMaxThreads / 32);   // the gap scan's byte table
+  uint32_t* bhist = reinterpret_cast<uint32_t*>(wrec + kMaxThreads / 32);    // byte values, kSmemHistCopies copies
+  uint8_t* btab = reinterpret_cast<uint8_t*>(bhist + kSmemHistCopies * kByteValues);   // the gap scan's byte table
 
   // the segment in hand, s_item[cur], and the next one, s_item[cur ^ 1],
   // claimed and looked up by warp 0 while the others mark (so no thread
   // waits on that lookup)
   __shared__ SegItem s_item[2];
   __shared__ uint32_t s_ctr;
-  __shared__ uint32_t s_vtab[32];      // bit b of a word -> 30*(b/8) + W30[b%8]
 
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t nthr = blockDim.x, nwarps = nthr >> 5;
 
   for (uint32_t i = tid; i < kSmemHistCopies * kSmemStride; i += nthr) shist[i] = 0;
-  if (tid < 32) s_vtab[tid] = 30u * (tid >> 3) + w30(tid & 7u);
-  for (uint32_t i = tid; i < kByteTabEntries; i += nthr) {
-    const uint64_t e = byte_gap_entry(i, false), od = byte_gap_entry(i, true);
-    btab[i] = make_uint4((uint32_t)e, (uint32_t)(e >> 32), (uint32_t)od, (uint32_t)(od >> 32));
-  }
+  for (uint32_t i = tid; i < kSmemHistCopies * kByteValues; i += nthr) bhist[i] = 0;
+  for (uint32_t x = tid; x < kByteValues; x += nthr)
+    btab[x] = x ? (uint8_t)((__ffs(x) - 1) | ((31 - __clz(x)) << 4)) : 0;
   if (tid == 0) s_ctr = 0;
   int cur_req = -1;
+  bool cur_gaps = false;
+  // Add the histograms to the current request's accumulators and clear them:
+  // the byte values give the primes, those 1 mod 3 and the gaps inside bytes
+  // (added to the first gap histogram).
+  auto flush = [&] {
+    ReqAccum* acc = prm.acc + cur_req;
+    for (uint32_t x = tid; x < kByteValues; x += nthr) {
+      uint32_t n = 0;
+#pragma unroll
+      for (int c = 0; c < kSmemHistCopies; ++c) { n += bhist[c * kByteValues + x]; bhist[c * kByteValues + x] = 0; }
+      // whole warps (kByteValues and the thread count are multiples of 32);
+      // sums of 32 products below 2^35 in two parts
+      const unsigned long long all = (unsigned long long)n * __popc(x);
+      const unsigned long long c1 = (unsigned long long)n * __popc(x & 0x2Bu);
+      const uint32_t all0 = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)all & 0xFFFFFFu);
+      const uint32_t all1 = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)(all >> 24));
+      const uint32_t c10 = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)c1 & 0xFFFFFFu);
+      const uint32_t c11 = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)(c1 >> 24));
+      if (lane == 0 && (all0 | all1)) {
+        atomicAdd(&acc->count, ((unsigned long long)all1 << 24) + all0);
+        atomicAdd(&acc->c31, ((unsigned long long)c11 << 24) + c10);
+      }
+      if (!n) continue;
+      for (uint32_t b = x; b & (b - 1u);) {
+        const uint32_t lo = __ffs(b) - 1u;
+        b &= b - 1u;
+        atomicAdd(&shist[(w30(__ffs(b) - 1u) - w30(lo)) >> 1], n);
+      }
+    }
+    __syncthreads();
+    for (uint32_t bn = tid; bn < (uint32_t)kSmemBins; bn += nthr) {
+      uint32_t s = 0;
+#pragma unroll
+      for (int c = 0; c < kSmemHistCopies; ++c) { s += shist[c * kSmemStride + bn]; shist[c * kSmemStride + bn] = 0; }
+      if (s && bn) atomicAdd(&acc->hist[bn], (unsigned long long)s);     // bin 0: the runs' first primes
+    }
+  };
 
   const uint64_t total_segs = prm.hdr->total_segs;
   const uint64_t item_end = prm.item_hi ? min(total_segs, prm.item_hi) : total_segs;
@@ -299,16 +372,12 @@ sieve_segments_kernel(const SieveParams prm) {
     const uint32_t np = S.np;
 
     if ((int)req != cur_req) {
-      if (cur_req >= 0) {                           // flush the previous request's bins
+      if (cur_req >= 0 && cur_gaps) {               // flush the previous request's counts
         __syncthreads();                            // after warp 0's last stitching gaps
-        for (uint32_t bn = tid; bn < (uint32_t)kSmemBins; bn += nthr) {
-          uint32_t s = 0;
-#pragma unroll
-          for (int c = 0; c < kSmemHistCopies; ++c) { s += shist[c * kSmemStride + bn]; shist[c * kSmemStride + bn] = 0; }
-          if (s) atomicAdd(&prm.acc[cur_req].hist[bn], (unsigned long long)s);
-        }
+        flush();
       }
       cur_req = (int)req;
+      cur_gaps = (S.rflags & kReqGaps) != 0;
     }
 
     // 1. presieve fill
@@ -614,115 +683,77 @@ sieve_segments_kernel(const SieveParams prm) {
       sk.req = req; sk.base = 30ull * k0;
       const uint32_t m41 = (k0 & 1ull) ? 0x99669966u : 0x66996699u;
       uint32_t first1 = 0, last1 = 0, cnt = 0, c41 = 0, c31 = 0, maxg = 0, maxgs = 0;
-      const bool gaps = (S.rflags & kReqGaps) != 0;
+      const bool gaps = uniform(S.rflags & kReqGaps) != 0;
       if (gaps) {
         // Byte by byte, four fixed steps per word, so the lanes of a warp
-        // stay in step whatever their primes: the gaps inside a wheel byte
-        // (2..28) come from the byte table and are summed in packed 8-bit
-        // counters (accE: gap/2 - 1 even, accO: odd), flushed warp-reduced
-        // into the shared histogram every kFlushWords words; the gap into a
-        // byte from the previous prime goes to the histogram directly, and
-        // to the rare path when it may be a new largest gap, a large gap or
-        // beyond the shared bins.  The run's first prime arrives as a gap
-        // from kNoPrev, which the rare path takes as "no gap, first prime".
-        constexpr uint32_t kNoPrev = 0x80000000u;
-        constexpr uint32_t kFlushWords = 15;      // 15 words * 4 bytes * 4 gaps of one size < 256
-        uint64_t accE = 0, accO = 0;
-        uint32_t pv = kNoPrev, thr = 0;
-        const uint32_t nsteps = run;              // the same for every lane
+        // stay in step whatever their primes.  A byte's value is counted in
+        // the byte histogram (its primes and the gaps inside it follow from
+        // that when the request is flushed), the gap into it from the
+        // previous prime in the gap histogram, and the largest such gap is
+        // kept as g << 23 | (2^23 - 1 - end), the earliest first on ties.
+        // (Before, a 16-byte table entry per byte brought the inner gaps as
+        // packed counters: 12 shared-memory wavefronts and 35 instructions
+        // per byte and warp, now 7 and 24: [9*10^11, 10^12) 16.5 -> 14.8 ms.)
+        // A run is walked prime by prime only where it holds a gap beyond the
+        // shared bins, or where no gap between bytes of the whole warp exceeds
+        // 28, the largest inside a byte.
+        const uint32_t hb = (uint32_t)__cvta_generic_to_shared(sk.shist);
+        const uint32_t bb = (uint32_t)__cvta_generic_to_shared(bhist + (warp % kSmemHistCopies) * kByteValues);
+        constexpr uint32_t kWlo = (uint32_t)kW30Packed, kWhi = (uint32_t)(kW30Packed >> 32);
+        constexpr uint32_t kEnd = (1u << 23) - 1u;
+        static_assert(30u * kMaxSegBytes < kEnd && 2 * kSmemBins < 512, "a gap and its end share 32 bits");
+        uint32_t fi = wbeg;                         // the run's first prime is its first "previous" one (gap 0)
+        while (fi < wend && !seg[fi]) ++fi;
+        uint32_t pv = fi < wend ? 120u * fi + word_value(__ffs(seg[fi]) - 1u) : 0u;
+        if (fi < wend) first1 = pv + 1u;
+        uint32_t top = 0;
+        const uint32_t nsteps = uniform(run);
+#pragma unroll 4
         for (uint32_t i = 0; i < nsteps; ++i) {
           const uint32_t wi = wbeg + i;
           const uint32_t w = wi < wend ? seg[wi] : 0u;
-          if (w) {
-            cnt += __popc(w);
-            c41 += __popc(w & m41);
-            c31 += __popc(w & 0x2B2B2B2Bu);
-            const uint32_t vb = 120u * wi;
+          c41 += __popc(w & m41);
+          const uint32_t vb = 120u * wi;
 #pragma unroll
-            for (uint32_t b = 0; b < 4; ++b) {
-              const uint32_t x = (w >> (8u * b)) & 0xFFu;
-              if (x) {
-                const uint4 t = btab[x];
-                accE += ((uint64_t)t.y << 32) | t.x;
-                accO += ((uint64_t)t.w << 32) | t.z;
-                const uint32_t v = vb + 30u * b + (t.y >> 24);
-                const uint32_t g = v - pv;
-                if (g <= thr) {
-                  atomicAdd(sk.shist + (g >> 1), 1u);
-                } else if (g & kNoPrev) {
-                  first1 = v + 1u;                  // the run's first prime
-                } else {
-                  const uint32_t bin = g >> 1;
-                  if (bin < (uint32_t)kSmemBins) atomicAdd(sk.shist + bin, 1u);
-                  else atomicAdd(&sk.acc->hist[bin < (uint32_t)kHistBins ? bin : kHistBins - 1], 1ull);
-                  if (g > maxg) { maxg = g; maxgs = pv; }
-                  if (g >= kLargeGap) {
-                    const unsigned idx = atomicAdd(sk.n_large, 1u);
-                    if (idx < sk.cap) {
-                      LargeGapRec r; r.pos = sk.base + v; r.gap = g; r.req = sk.req;
-                      sk.large[idx] = r;
-                    }
-                  }
-                  thr = min(maxg, kLargeGap - 1u);
-                }
-                pv = vb + 30u * b + (t.w >> 24);
-              }
-            }
-          }
-          if ((i + 1u) % kFlushWords == 0u || i + 1u == nsteps) {
-            // 16-bit pairs of the 8-bit counters, summed over the warp; lane
-            // k < 7 adds pair k (bins 2k+1, 2k+3 from accE; k >= 4 accO)
-            const uint32_t eL = (uint32_t)accE, eH = (uint32_t)(accE >> 32);
-            const uint32_t oL = (uint32_t)accO, oH = (uint32_t)(accO >> 32);
-            const uint32_t q0 = __reduce_add_sync(0xFFFFFFFFu, __byte_perm(eL, 0u, 0x5150));   // bins 1, 3
-            const uint32_t q1 = __reduce_add_sync(0xFFFFFFFFu, __byte_perm(eL, 0u, 0x5352));   // bins 5, 7
-            const uint32_t q2 = __reduce_add_sync(0xFFFFFFFFu, __byte_perm(eH, 0u, 0x5150));   // bins 9, 11
-            const uint32_t q3 = __reduce_add_sync(0xFFFFFFFFu, __byte_perm(eH, 0u, 0x4442));   // bin 13
-            const uint32_t q4 = __reduce_add_sync(0xFFFFFFFFu, __byte_perm(oL, 0u, 0x5150));   // bins 2, 4
-            const uint32_t q5 = __reduce_add_sync(0xFFFFFFFFu, __byte_perm(oL, 0u, 0x5352));   // bins 6, 8
-            const uint32_t q6 = __reduce_add_sync(0xFFFFFFFFu, __byte_perm(oH, 0u, 0x5150));   // bins 10, 12
-            const uint32_t q7 = __reduce_add_sync(0xFFFFFFFFu, __byte_perm(oH, 0u, 0x4442));   // bin 14
-            accE = 0;
-            accO = 0;
-            if (lane < 8u) {
-              const uint32_t q = lane == 0 ? q0 : lane == 1 ? q1 : lane == 2 ? q2 : lane == 3 ? q3
-                               : lane == 4 ? q4 : lane == 5 ? q5 : lane == 6 ? q6 : q7;
-              // pair k of accE holds bins 4k'+1.. : lane 0 -> 1,3; 1 -> 5,7; 2 -> 9,11; 3 -> 13
-              // accO: lane 4 -> 2,4; 5 -> 6,8; 6 -> 10,12; 7 -> 14
-              const uint32_t b0 = lane < 4u ? 4u * lane + 1u : 4u * (lane - 4u) + 2u;
-              if (q & 0xFFFFu) atomicAdd(sk.shist + b0, q & 0xFFFFu);
-              if (q >> 16) atomicAdd(sk.shist + b0 + 2u, q >> 16);
+          for (uint32_t b = 0; b < 4; ++b) {
+            const uint32_t x = (w >> (8u * b)) & 0xFFu;
+            if (x) {
+              const uint32_t e = btab[x];
+              count_one(bb + 4u * x);
+              const uint32_t r = __byte_perm(kWlo, kWhi, e);      // W30 of the lowest, the highest bit
+              const uint32_t v = vb + 30u * b + (r & 0xFFu);
+              const uint32_t g = min(v - pv, 2u * (uint32_t)kSmemBins);
+              pv = vb + 30u * b + ((r >> 8) & 0xFFu);
+              count_one(hb + 2u * g);
+              top = max(top, (g << 23) + (kEnd - v));
             }
           }
         }
-        // A largest gap inside a byte (at most 28) is not tracked above:
-        // where no gap between bytes exceeds 28, the run is walked prime by
-        // prime for its exact largest gap (the earliest one on ties).
-        if (first1 && maxg <= 28u) {
-          maxg = 0; maxgs = 0;
-          uint32_t q = first1 - 1u;
-          for (uint32_t wi = wbeg; wi < wend; ++wi) {
-            uint32_t w = seg[wi];
-            const uint32_t vb = 120u * wi;
-            while (w) {
-              const uint32_t v = vb + s_vtab[__ffs(w) - 1];
-              w &= w - 1u;
-              if (v - q > maxg) { maxg = v - q; maxgs = q; }
-              q = v;
-            }
-          }
+        if (first1) {
+          last1 = pv + 1u;
+          maxg = top >> 23;
+          maxgs = kEnd - (top & kEnd) - maxg;
         }
-        last1 = first1 ? pv + 1u : 0u;
+        const uint32_t wmax = __reduce_max_sync(0xFFFFFFFFu, maxg);
+        if (first1 && (wmax <= 28u || maxg >= 2u * (uint32_t)kSmemBins)) {
+          const uint2 m = walk_run(sk, seg, wbeg, wend);
+          maxg = m.x;
+          maxgs = m.y;
+        }
       } else {
+        uint32_t lastw = 0, lasti = 0;
         for (uint32_t wi = wbeg; wi < wend; ++wi) {
           const uint32_t w = seg[wi];
-          if (!w) continue;
           cnt += __popc(w);
           c41 += __popc(w & m41);
           c31 += __popc(w & 0x2B2B2B2Bu);
-          const uint32_t vb = 120u * wi;
-          if (!first1) first1 = vb + s_vtab[__ffs(w) - 1] + 1u;
-          last1 = vb + s_vtab[31 - __clz(w)] + 1u;
+          if (w) { lastw = w; lasti = wi; }
+        }
+        if (lastw) {
+          last1 = 120u * lasti + word_value(31u - __clz(lastw)) + 1u;
+          uint32_t wi = wbeg;
+          while (!seg[wi]) ++wi;
+          first1 = 120u * wi + word_value(__ffs(seg[wi]) - 1u) + 1u;
         }
       }
       // lane stitching: previous lane's last prime (values grow with the lane)
@@ -780,11 +811,11 @@ sieve_segments_kernel(const SieveParams prm) {
           sr.last = run1 ? sk.base + run1 - 1u : 0;
           sr.max_gap = gm;
           sr.max_gap_start = gm ? sk.base + gs : 0;
-          sr.count = tc;
+          sr.pad = 0;
           prm.segs[item] = sr;
-          if (tc) {
+          if (t41) atomicAdd(&sk.acc->c41, (unsigned long long)t41);
+          if (tc) {                                   // with gaps: from the byte histogram
             atomicAdd(&sk.acc->count, (unsigned long long)tc);
-            atomicAdd(&sk.acc->c41, (unsigned long long)t41);
             atomicAdd(&sk.acc->c31, (unsigned long long)t31);
           }
         }
@@ -792,14 +823,7 @@ sieve_segments_kernel(const SieveParams prm) {
     }
   }
   __syncthreads();
-  if (cur_req >= 0) {
-    for (uint32_t bn = tid; bn < (uint32_t)kSmemBins; bn += nthr) {
-      uint32_t s = 0;
-#pragma unroll
-      for (int c = 0; c < kSmemHistCopies; ++c) s += shist[c * kSmemStride + bn];
-      if (s) atomicAdd(&prm.acc[cur_req].hist[bn], (unsigned long long)s);
-    }
-  }
+  if (cur_req >= 0 && cur_gaps) flush();
 }
 
 // One CTA per request: seeds 2, 3, 5, gaps across segment boundaries, the
@@ -1114,9 +1138,10 @@ __global__ void zero_kernel(ZeroSpan z0, ZeroSpan z1, ZeroSpan z2) {
 // host-side launchers (called by the engine)
 // ---------------------------------------------------------------------------
 size_t sieve_smem_bytes(uint32_t seg_bytes, uint32_t /*threads*/) {
-  // segment, histogram copies, warp records (room for 32 warps), byte table
+  // segment, gap histogram copies, warp records (room for 32 warps), byte
+  // histogram copies, byte table
   return (size_t)seg_bytes + sizeof(uint32_t) * kSmemHistCopies * kSmemStride +
-         sizeof(WarpRec) * (kMaxThreads / 32) + sizeof(uint4) * kByteTabEntries;
+         sizeof(WarpRec) * (kMaxThreads / 32) + sizeof(uint32_t) * kSmemHistCopies * kByteValues + kByteValues;
 }
 
 size_t sieve_static_smem_bytes() {
