@@ -212,6 +212,37 @@ uint32_t Engine::wheel_begin(uint32_t seg_bytes, uint32_t tier_split) const {
   return wheel_begin_index(seg_bytes, tier_split, [&](uint32_t p) { return index_of(p); });
 }
 
+ReqDesc Engine::describe(uint64_t a, uint64_t b, uint32_t rflags, const Config& c) const {
+  ReqDesc r{};
+  r.a = a;
+  r.b = b;
+  r.rflags = rflags;
+  r.k_lo = a / 30;
+  r.k_hi = (b + 29) / 30;
+  r.seg_bytes = c.seg_bytes;
+  r.nseg = (r.k_hi - r.k_lo + c.seg_bytes - 1) / c.seg_bytes;
+  r.nprimes = primes_below_sq(b);
+  r.tier_split = index_of(c.tier_split);
+  r.tier_wheel = wheel_begin(c.seg_bytes, r.tier_split);
+  r.bucket_idx = r.nprimes;
+  return r;
+}
+
+SieveParams Engine::table_params() const {
+  SieveParams prm{};
+  prm.P = dP.as<uint32_t>();
+  prm.M = dM.as<uint64_t>();
+  prm.R = dR.as<uint32_t>();
+  prm.W = dW.as<WheelEntry>();
+  prm.Woff = dWoff.as<uint32_t>();
+  prm.ntab = (uint32_t)hP.size();
+  for (int t = 0; t < kTiles; ++t) {
+    prm.tile[t] = tile[t].as<uint32_t>();
+    prm.tile_stride16[t] = tile_copy_stride(tile_period(t), kMaxSegBytes) / 16;
+  }
+  return prm;
+}
+
 Config Engine::tuned_for(uint64_t a, uint64_t b, bool batch) const {
   Config c = cfg;
   if (!cfg.auto_tune) return c;
@@ -232,7 +263,9 @@ Config Engine::tuned_for(uint64_t a, uint64_t b, bool batch) const {
   }
   // Alone, a range should fill the GPU in whole waves: the segment shrinks
   // until the segments come in full waves of one CTA per SM (not below 16 KiB,
-  // where the per-prime setup dominates).  In a batch other ranges fill the
+  // where the per-prime setup dominates; with at most 3400 sieving primes not
+  // below 4 KiB: a call over [0, 10^7) takes 34.5 us there, 38.9 with 16 KiB,
+  // one of width 10^7 at 10^12 73 and 43).  In a batch other ranges fill the
   // GPU, so the largest segment is the cheapest.
   if (batch) {
     s = cfg.seg_bytes;
@@ -240,7 +273,7 @@ Config Engine::tuned_for(uint64_t a, uint64_t b, bool batch) const {
     const uint64_t g = (uint64_t)sm_count * cfg.ctas_per_sm;
     const uint64_t waves = (bytes + g * s - 1) / (g * s);
     uint64_t want = (bytes + waves * g - 1) / (waves * g);
-    want = std::max<uint64_t>(want, 16384);
+    want = std::max<uint64_t>(want, b <= 1000000000ull ? 4096 : 16384);
     s = (uint32_t)std::min<uint64_t>(s, (want + 127) & ~127ull);
   }
   c.seg_bytes = s;
@@ -448,13 +481,7 @@ void Plan::load_requests(uint32_t n, const uint64_t* a, const uint64_t* b, uint3
     double cost = 0;
     if (b[i] > a[i]) {
       const Config c = E.tuned_for(a[i], b[i], many);
-      r.k_lo = a[i] / 30;
-      r.k_hi = (b[i] + 29) / 30;
-      r.seg_bytes = c.seg_bytes;
-      r.nseg = (r.k_hi - r.k_lo + c.seg_bytes - 1) / c.seg_bytes;
-      r.nprimes = E.primes_below_sq(b[i]);
-      r.tier_split = E.index_of(c.tier_split);
-      r.tier_wheel = E.wheel_begin(c.seg_bytes, r.tier_split);
+      r = E.describe(a[i], b[i], r.rflags, c);
       smax = std::max(smax, c.seg_bytes);
       // per segment: fill and scan grow with the bytes, setup with the primes
       cost = (double)r.nseg * ((double)c.seg_bytes + 24.0 * r.nprimes);
@@ -564,19 +591,10 @@ void Plan::load_requests(uint32_t n, const uint64_t* a, const uint64_t* b, uint3
   const uint64_t gcap = (uint64_t)E.sm_count * E.cfg.ctas_per_sm;
   grid = (uint32_t)(cap_req ? gcap : std::min<uint64_t>(total_segs, gcap));
 
+  prm = E.table_params();
   prm.reqs = dreqs();
   prm.hdr = hdr.as<BatchHdr>();
   prm.queue = &dctl()->queue;
-  prm.P = E.dP.as<uint32_t>();
-  prm.M = E.dM.as<uint64_t>();
-  prm.R = E.dR.as<uint32_t>();
-  prm.W = E.dW.as<WheelEntry>();
-  prm.Woff = E.dWoff.as<uint32_t>();
-  prm.ntab = (uint32_t)E.hP.size();
-  for (int t = 0; t < kTiles; ++t) {
-    prm.tile[t] = E.tile[t].as<uint32_t>();
-    prm.tile_stride16[t] = tile_copy_stride(tile_period(t), kMaxSegBytes) / 16;
-  }
   prm.seg_bytes = seg_max;
   prm.segs = segs.as<SegRec>();
   prm.acc = acc.as<ReqAccum>();
@@ -788,8 +806,79 @@ uint64_t Plan::algorithmic_clears() const {
   return total;
 }
 
+// Bytes of the segments that several CTAs share in one run (their merged words).
+constexpr uint64_t kSoloMergeBytes = 4u << 20;
+// Sieving primes per CTA down to which a segment's primes are split (a call of
+// width 10^4 at 10^9: 34.8 / 30.3 / 30.7 us with 2048 / 512 / 128; Context(10^7)
+// 38.7 / 38.9 / 37.3).
+constexpr uint32_t kSoloSlicePrimes = 256;
+// Above this many primes per CTA past the bucket split, lists are cheaper: a
+// call of width 10^7 at 9*10^13 (92 000 per CTA) takes 75 us without and 113
+// with them, of 10^8 at 10^12 (59 000) 84 and 92; of 10^8 at 9*10^13 (610 000)
+// the fill is far cheaper.
+constexpr uint32_t kSoloListPrimes = 100000;
+constexpr uint32_t kSoloLargeCap = 1u << 14;
+
+const ReqResult* Engine::run_solo(uint64_t a, uint64_t b, std::vector<LargeGapRec>* lg, bool gaps) {
+  if (b <= a || b > kMaxB) return nullptr;
+  ensure_table(isqrt_u64(b - 1));
+  const Config c = tuned_for(a, b, false);
+  const ReqDesc r = describe(a, b, gaps ? kReqGaps : 0u, c);
+  const uint64_t ctas = std::min<uint64_t>((uint64_t)sm_count * cfg.ctas_per_sm, kSoloMaxSegs);
+  if (r.nseg > ctas) return nullptr;
+  uint64_t slices = 1;
+  if (r.nseg * r.seg_bytes <= kSoloMergeBytes)
+    slices = std::max<uint64_t>(1, std::min<uint64_t>(ctas / r.nseg, r.nprimes / kSoloSlicePrimes));
+  const BucketPlan bp = bucket_plan(c, b, r.nprimes, r.nseg, r.seg_bytes);
+  if (bp.cap && (!cfg.auto_tune || (r.nprimes - bp.bucket_idx) / slices > kSoloListPrimes)) return nullptr;
+
+  if (!solo.clean) {
+    solo.ctl.reserve(sizeof(SoloCtl));
+    solo.acc.reserve(sizeof(ReqAccum));
+    solo.segs.reserve(sizeof(SegRec) * kSoloMaxSegs);
+    solo.merge.reserve(kSoloMergeBytes);
+    solo.large.reserve(sizeof(LargeGapRec) * kSoloLargeCap);
+    solo.out.reserve(sizeof(SoloResult));
+    check_cuda(cudaMemsetAsync(solo.ctl.ptr, 0, sizeof(SoloCtl), stream), "solo control");
+    check_cuda(cudaMemsetAsync(solo.acc.ptr, 0, sizeof(ReqAccum), stream), "solo accumulators");
+    check_cuda(cudaMemsetAsync(solo.merge.ptr, 0xFF, kSoloMergeBytes, stream), "solo words");
+  }
+  SieveParams prm = table_params();
+  prm.seg_bytes = r.seg_bytes;
+  prm.segs = solo.segs.as<SegRec>();
+  prm.acc = solo.acc.as<ReqAccum>();
+  prm.large = solo.large.as<LargeGapRec>();
+  prm.n_large = &solo.ctl.as<SoloCtl>()->n_large;
+  prm.large_cap = kSoloLargeCap;
+  prm.solo = r;
+  prm.slices = (uint32_t)slices;
+  const uint64_t rows = ((uint64_t)r.nprimes + kWheelRow - 1) / kWheelRow * kWheelRow;
+  prm.low_k = r.nprimes ? hP[std::min<uint64_t>(rows, hP.size()) - 1] / 30u + 1u : 0u;
+  prm.keep0 = first_word_mask(r);
+  prm.keepl = last_word_mask(r, (uint32_t)(r.k_hi - r.k_lo - (r.nseg - 1) * r.seg_bytes));
+  prm.merge = solo.merge.as<uint32_t>();
+  prm.ctl = solo.ctl.as<SoloCtl>();
+  prm.out = static_cast<SoloResult*>(solo.out.ptr);
+  solo.clean = false;                        // until the run has ended well
+  check_cuda(launch_solo(prm, cfg.threads, stream), "solo_kernel");
+  check_cuda(cudaStreamSynchronize(stream), "sieve run");
+  solo.clean = true;
+  const SoloResult* out = static_cast<const SoloResult*>(solo.out.ptr);
+  if (lg) {
+    if (out->n_large > kSoloLargeCap)
+      throw Error(VOSS_ERR_INTERNAL, "large-gap buffer overflow (" + std::to_string(out->n_large) + " gaps)");
+    lg->resize(out->n_large);
+    if (out->n_large)
+      check_cuda(cudaMemcpy(lg->data(), solo.large.ptr, sizeof(LargeGapRec) * out->n_large, cudaMemcpyDeviceToHost),
+                 "large gaps");
+  }
+  return &out->res;
+}
+
 const ReqResult* Engine::run(uint32_t n, const uint64_t* a, const uint64_t* b,
                              std::vector<LargeGapRec>* lg, bool gaps, bool share) {
+  if (n == 1)
+    if (const ReqResult* r = run_solo(a[0], b[0], lg, gaps)) return r;
   std::vector<uint32_t> rf(n, gaps ? kReqGaps : 0u);
   struct Unshare { Plan& p; ~Unshare() { p.share = false; } } unshare{scratch};
   scratch.share = share && !lg && n > 1;

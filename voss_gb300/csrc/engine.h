@@ -242,6 +242,13 @@ class Engine {
 
   // Scratch plan reused by the synchronous entry points.
   Plan scratch;
+  // The one-launch form for a lone range (solo_kernel): its device buffers,
+  // left clean by every run, and the result in host memory.
+  struct Solo {
+    DevBuf ctl, acc, segs, merge, large;
+    HostPinned out;
+    bool clean = false;
+  } solo;
   // Buffers of the synchronous calls that read a wheel bitmap (in_range,
   // Sophie Germain, Goldbach), kept between calls up to a bound (guarded by
   // mu like scratch).
@@ -261,6 +268,12 @@ class Engine {
                          uint32_t seg_bytes) const;
   std::vector<TuneEntry> tuning;
 
+  // The device request of [a, b) under configuration c, without its place in
+  // a batch or lists.
+  ReqDesc describe(uint64_t a, uint64_t b, uint32_t rflags, const Config& c) const;
+  // Kernel parameters with the tables filled in.
+  SieveParams table_params() const;
+
   // Run ranges synchronously on the engine stream.  share: overlapping
   // ranges sieve their common integers once (not with large-gap output).
   const ReqResult* run(uint32_t n, const uint64_t* a, const uint64_t* b,
@@ -271,6 +284,8 @@ class Engine {
   Engine() = default;
   void init();
   void build_tiles();
+  // A lone range in one launch, or null where that form does not fit it.
+  const ReqResult* run_solo(uint64_t a, uint64_t b, std::vector<LargeGapRec>* large, bool gaps);
 };
 
 void smem_peaks(Engine& E, double* ldst_gbs, double* atomic_gbs);
@@ -290,6 +305,7 @@ size_t sieve_smem_bytes(uint32_t seg_bytes, uint32_t threads);
 size_t sieve_static_smem_bytes();      // the sieve kernel's static shared memory
 cudaError_t launch_sieve(const SieveParams& prm, uint32_t grid, uint32_t threads,
                          cudaStream_t stream);
+cudaError_t launch_solo(const SieveParams& prm, uint32_t threads, cudaStream_t stream);
 cudaError_t launch_bucket_fill(const FillParams& fp, uint32_t grid, cudaStream_t stream);
 uint32_t bucket_fill_ctas_per_sm();      // resident fill CTAs per SM (occupancy query, cached)
 // Cut a batch's ranges at every endpoint into the disjoint pieces some range

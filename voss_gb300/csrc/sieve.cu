@@ -203,6 +203,16 @@ struct SegItem {
   uint32_t and0, or0, keep0, keepl;
 };
 
+// What follows from a work item's request R: the tiers, the flags and the edge
+// masks (keep0 and keepl where the segment is the first or the last).
+__device__ __forceinline__ void set_item(SegItem& d, const ReqDesc& R, uint32_t keep0, uint32_t keepl) {
+  d.split = R.tier_split; d.wheel = R.tier_wheel; d.rflags = R.rflags;
+  d.and0 = d.k0 == 0 ? ~1u : ~0u;                                        // 1 is not prime
+  d.or0 = d.k0 < 3 ? (uint32_t)(kTilePrimeBits >> (8u * d.k0)) : 0u;     // the tile primes are
+  d.keep0 = keep0;                                                       // numbers below a
+  d.keepl = keepl;                                                       // numbers from b on
+}
+
 // Number of leading i in [0, n) for which pred(i) holds (pred holds on a
 // prefix), by a 32-ary search of one warp: each step probes 32 evenly spaced
 // points, so about log32(n) dependent loads instead of log2(n).
@@ -259,24 +269,7 @@ __device__ __noinline__ void claim_item(unsigned long long* queue, const ReqDesc
     }
     d.item = item; d.valid = 1;
     d.req = r; d.k0 = k0; d.nbytes = nb; d.np = a;
-    d.split = R.tier_split; d.wheel = R.tier_wheel; d.rflags = R.rflags;
-    uint32_t and0 = ~0u, or0 = 0u, keep0 = ~0u, keepl = ~0u;
-    if (k0 == 0) and0 = ~1u;                               // 1 is not prime
-    if (k0 < 3) or0 = (uint32_t)(kTilePrimeBits >> (8u * k0));   // the tile primes are
-    if (si == 0) {                                         // numbers below a
-      for (uint32_t o = 0; o < 8; ++o)
-        if (30ull * k0 + w30(o) < R.a) keep0 &= ~(1u << o);
-    }
-    if (k0 + nb == R.k_hi) {                               // numbers from b on
-      const uint32_t lb = nb - 1;
-      uint32_t m = 0;
-      for (uint32_t o = 0; o < 8; ++o)
-        if (30ull * (k0 + lb) + w30(o) >= R.b) m |= 1u << o;
-      keepl = ~(m << ((lb & 3u) << 3));
-      const uint32_t rem = nb & 3u;                        // bytes past the end
-      if (rem) keepl &= (1u << (rem << 3)) - 1u;
-    }
-    d.and0 = and0; d.or0 = or0; d.keep0 = keep0; d.keepl = keepl;
+    set_item(d, R, si == 0 ? first_word_mask(R) : ~0u, k0 + nb == R.k_hi ? last_word_mask(R, nb) : ~0u);
   }
 }
 
@@ -288,8 +281,112 @@ struct WarpRec {
   uint32_t pad;
 };
 
-__global__ void __launch_bounds__(kMaxThreads, 1)
-sieve_segments_kernel(const SieveParams prm) {
+__device__ __forceinline__ SegRec seg_rec(const SegRec* s) {
+  const ulonglong2 a = __ldcg(reinterpret_cast<const ulonglong2*>(s));
+  const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2*>(s) + 1);
+  SegRec r;
+  r.first = a.x; r.last = a.y; r.max_gap_start = b.x;
+  r.max_gap = (uint32_t)b.y; r.pad = 0;
+  return r;
+}
+static_assert(sizeof(SegRec) == 32 && alignof(SegRec) == 16, "read as two 16-byte halves");
+
+// Shared memory of finalize_request: 32-bit words.
+constexpr uint32_t kFinalWords = kHistBins + 1u + 8u * 32u;
+
+// The whole CTA finishes request r: seeds 2, 3, 5, gaps across segment
+// boundaries, the largest gap, and the final counts (the reference's host-side
+// conventions, context.cu:321-322,462-524, restated for a half-open [a, b)).
+// Records and accumulators are read past L1: other CTAs of the same launch may
+// have written them.  kClean: the accumulators are left at zero.
+template <bool kClean>
+__device__ __forceinline__ void finalize_request(const ReqDesc& R, uint32_t r, const SegRec* S, ReqAccum* A,
+                                                 LargeGapRec* large, unsigned int* n_large, uint32_t large_cap,
+                                                 ReqResult* O, uint32_t* tmp) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  uint32_t* const joins = tmp;                       // gaps between segments and seeds, per bin
+  uint64_t* const part = reinterpret_cast<uint64_t*>(tmp + kHistBins + 1);     // per warp: four values
+  const bool in2 = R.a <= 2 && 2 < R.b, in3 = R.a <= 3 && 3 < R.b, in5 = R.a <= 5 && 5 < R.b;
+  const uint64_t seed_first = in2 ? 2 : in3 ? 3 : in5 ? 5 : 0;
+  const uint64_t seed_last = in5 ? 5 : in3 ? 3 : in2 ? 2 : 0;
+  const bool gaps = (R.rflags & kReqGaps) != 0;
+  uint64_t wc = 0, a41 = 0, a31 = 0;
+  if (tid == 0) { wc = __ldcg(&A->count); a41 = __ldcg(&A->c41); a31 = __ldcg(&A->c31); }
+  for (uint32_t b = tid; b < (uint32_t)kHistBins; b += blockDim.x) joins[b] = 0;
+  __syncthreads();
+
+  uint64_t bg = 0, bs = 0, first = ~0ull, last = 0;
+  auto consider = [&](uint64_t g, uint64_t st) {
+    if (g > bg || (g == bg && g && st < bs)) { bg = g; bs = st; }
+  };
+  if (tid == 0 && gaps) {
+    if (in2 && in3) { atomicAdd(&joins[0], 1u); consider(1, 2); }
+    if (in3 && in5) { atomicAdd(&joins[1], 1u); consider(2, 3); }
+  }
+  for (uint64_t i = tid; i < R.nseg; i += blockDim.x) {
+    const SegRec s = seg_rec(S + i);
+    if (!s.first) continue;
+    first = s.first < first ? s.first : first;
+    last = s.last > last ? s.last : last;
+    if (!gaps) continue;
+    if (s.max_gap) consider(s.max_gap, s.max_gap_start);
+    uint64_t prev = 0;
+    for (uint64_t j = i; j-- > 0;) {
+      if (__ldcg(&S[j].first)) { prev = __ldcg(&S[j].last); break; }
+    }
+    if (!prev) prev = seed_last;
+    if (!prev) continue;
+    const uint64_t g = s.first - prev;
+    const uint64_t bin = g >> 1;
+    atomicAdd(&joins[bin < (uint64_t)kHistBins ? bin : kHistBins - 1], 1u);
+    consider(g, prev);
+    if (g >= kLargeGap) {
+      const unsigned idx = atomicAdd(n_large, 1u);
+      if (idx < large_cap) {
+        LargeGapRec lr; lr.pos = s.first; lr.gap = (uint32_t)g; lr.req = r;
+        large[idx] = lr;
+      }
+    }
+  }
+  // the largest gap (the earliest on ties), the first and the last prime
+  auto fold = [&](uint64_t g2, uint64_t s2, uint64_t f2, uint64_t l2) {
+    consider(g2, s2);
+    first = f2 < first ? f2 : first;
+    last = l2 > last ? l2 : last;
+  };
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const uint64_t g2 = __shfl_down_sync(0xFFFFFFFFu, bg, d), s2 = __shfl_down_sync(0xFFFFFFFFu, bs, d);
+    const uint64_t f2 = __shfl_down_sync(0xFFFFFFFFu, first, d), l2 = __shfl_down_sync(0xFFFFFFFFu, last, d);
+    fold(g2, s2, f2, l2);
+  }
+  if (lane == 0) { part[4 * warp] = bg; part[4 * warp + 1] = bs; part[4 * warp + 2] = first; part[4 * warp + 3] = last; }
+  __syncthreads();
+  for (uint32_t b = tid; b < (uint32_t)kHistBins; b += blockDim.x) {
+    O->hist[b] = __ldcg(&A->hist[b]) + joins[b];
+    if (kClean) A->hist[b] = 0;
+  }
+  if (tid == 0) {
+    for (uint32_t w = 1; w < blockDim.x >> 5; ++w) fold(part[4 * w], part[4 * w + 1], part[4 * w + 2], part[4 * w + 3]);
+    const uint64_t ns = (uint64_t)in2 + in3 + in5;
+    const uint64_t count = wc + ns;
+    O->count = count;
+    O->c41 = a41 + (in5 ? 1 : 0);
+    O->c43 = (wc - a41) + (in3 ? 1 : 0);
+    O->c31 = a31;
+    O->c32 = (wc - a31) + (in2 ? 1 : 0) + (in5 ? 1 : 0);
+    O->first = seed_first ? seed_first : first != ~0ull ? first : 0;
+    O->last = last ? last : seed_last;
+    O->max_gap = bg;
+    O->max_gap_start = bg ? bs : 0;
+    O->num_gaps = count ? count - 1 : 0;
+    if (kClean) A->count = A->c41 = A->c31 = 0;
+  }
+}
+
+// kSolo: the one-launch form for a lone request, see solo_kernel.
+template <bool kSolo>
+__device__ __forceinline__ void sieve_body(const SieveParams& prm) {
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* seg = smem;
   const uint32_t sseg = (uint32_t)__cvta_generic_to_shared(seg);
@@ -351,11 +448,29 @@ sieve_segments_kernel(const SieveParams prm) {
     }
   };
 
-  const uint64_t total_segs = prm.hdr->total_segs;
-  const uint64_t item_end = prm.item_hi ? min(total_segs, prm.item_hi) : total_segs;
-  const uint32_t nreq = prm.hdr->nreq;
-  uint32_t cur = 0;
-  if (warp == 0) claim_item(prm.queue, prm.reqs, prm.P, prm.bcount, prm.item_lo, item_end, prm.list_seg0, nreq, s_item[0], lane);
+  uint64_t item_end = 0;
+  uint32_t nreq = 1, cur = 0;
+  // solo: this CTA's segment and its share of the segment's units
+  const uint32_t slices = kSolo ? prm.slices : 1u;
+  const uint32_t slice = kSolo ? blockIdx.x % slices : 0u;
+  if constexpr (kSolo) {
+    if (tid == 0) {
+      const ReqDesc& R = prm.solo;
+      SegItem& d = s_item[0];
+      const uint32_t si = blockIdx.x / slices;
+      d.k0 = R.k_lo + (uint64_t)si * R.seg_bytes;
+      d.nbytes = (uint32_t)min((uint64_t)R.seg_bytes, R.k_hi - d.k0);
+      d.item = si; d.valid = 1; d.req = 0; d.np = R.nprimes; d.bcnt = 0; d.bbase = 0;
+      set_item(d, R, si == 0 ? prm.keep0 : ~0u, si + 1u == (uint32_t)R.nseg ? prm.keepl : ~0u);
+      s_item[1].valid = 0;
+    }
+  } else {
+    const uint64_t total_segs = prm.hdr->total_segs;
+    item_end = prm.item_hi ? min(total_segs, prm.item_hi) : total_segs;
+    nreq = prm.hdr->nreq;
+    if (warp == 0)
+      claim_item(prm.queue, prm.reqs, prm.P, prm.bcount, prm.item_lo, item_end, prm.list_seg0, nreq, s_item[0], lane);
+  }
   __syncthreads();
   // Three barriers per segment: after the fill, after the marking, before
   // the warps are stitched.  No thread reads the segment after the last one,
@@ -380,8 +495,9 @@ sieve_segments_kernel(const SieveParams prm) {
       cur_gaps = (S.rflags & kReqGaps) != 0;
     }
 
-    // 1. presieve fill
-    {
+    // 1. presieve fill, of all words or (solo, after the slices are merged)
+    //    into what the slices left
+    auto fill = [&](const uint32_t* merged) {
       // copy (phase mod 16) of each tile holds the phase on a 16-byte boundary
       uint32_t toff[kTiles];                       // 16-byte units from each tile's start
 #pragma unroll
@@ -399,8 +515,18 @@ sieve_segments_kernel(const SieveParams prm) {
           const uint4 y = __ldg(reinterpret_cast<const uint4*>(prm.tile[t]) + toff[t] + v);
           x.x &= y.x; x.y &= y.y; x.z &= y.z; x.w &= y.w;
         }
+        if (kSolo && merged) {
+          const uint4 y = __ldcg(reinterpret_cast<const uint4*>(merged) + v);
+          x.x &= y.x; x.y &= y.y; x.z &= y.z; x.w &= y.w;
+        }
         seg4[v] = x;
       }
+    };
+    if (kSolo && slices > 1u) {
+      const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
+      for (uint32_t v = tid; v < (nbytes + 15u) >> 4; v += nthr) reinterpret_cast<uint4*>(seg)[v] = ones;
+    } else {
+      fill(nullptr);
     }
     __syncthreads();
 
@@ -431,7 +557,7 @@ sieve_segments_kernel(const SieveParams prm) {
       // primes per unit, 2^wlog: claiming a unit costs about as much as
       // marking 32 primes, but every warp should get several units
       uint32_t wlog = 5;
-      while (wlog < kWheelUnitLog2Max && mend + (256u << wlog) <= unp) ++wlog;
+      while (wlog < kWheelUnitLog2Max && mend + ((256u * slices) << wlog) <= unp) ++wlog;
       uint32_t wincl = (wend - wbeg + (1u << wlog) - 1u) >> wlog;
 #pragma unroll
       for (int d = 1; d < 8; d <<= 1) {
@@ -444,7 +570,7 @@ sieve_segments_kernel(const SieveParams prm) {
       const uint32_t k0s = uniform((uint32_t)(k0 >> 10)), k0l = uniform((uint32_t)k0);
       const uint32_t bcnt = uniform(S.bcnt);
       const uint64_t bbase = S.bbase;
-      if (warp == 0)                                // overlaps the marking
+      if (!kSolo && warp == 0)                      // overlaps the marking
         claim_item(prm.queue, prm.reqs, prm.P, prm.bcount, prm.item_lo, item_end, prm.list_seg0, nreq,
                    s_item[cur ^ 1u], lane);
       const uint32_t nunits = nscan + (bcnt + kBucketUnit - 1) / kBucketUnit;
@@ -454,6 +580,7 @@ sieve_segments_kernel(const SieveParams prm) {
         uint32_t u = 0;
         if (lane == 0) u = atomicAdd(&s_ctr, 1u);
         u = uniform(u);
+        if (kSolo) u = u * slices + slice;
         if (u >= nunits) break;
         if (u < nsmall) {
           const bool cst = u < kConstPrimes;
@@ -649,7 +776,26 @@ sieve_segments_kernel(const SieveParams prm) {
     // prime that sieves it (p*p < 30 (k0 + nbytes) and p >= 30 k0 need k0 <=
     // 86; the rounding to a row adds primes of less than 3840): there they are
     // set again.  This spares every hit a p*p test.
-    if (k0 < 128u) {
+    // (Solo sieves every segment with the request's last prime; its host gives
+    // the bound.)
+    if (kSolo && slices > 1u) {
+      // merge the slices; the last one to arrive goes on
+      uint32_t* const words = prm.merge + (uint64_t)item * (prm.seg_bytes >> 2);
+      for (uint32_t w = tid; w < nwords; w += nthr)
+        if (seg[w] != ~0u) atomicAnd(words + w, seg[w]);
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) s_ctr = atomicAdd(&prm.ctl->seg_done[item], 1u);
+      __syncthreads();
+      if (s_ctr != slices - 1u) return;
+      __threadfence();
+      fill(words);
+      __syncthreads();
+      uint4* const w4 = reinterpret_cast<uint4*>(words);
+      for (uint32_t v = tid; v < (nbytes + 15u) >> 4; v += nthr) w4[v] = make_uint4(~0u, ~0u, ~0u, ~0u);
+      if (tid == 0) prm.ctl->seg_done[item] = 0;
+    }
+    if (k0 < (kSolo ? prm.low_k : 128u)) {
       const uint32_t nset = min((np + kWheelRow - 1u) / kWheelRow * kWheelRow, prm.ntab);
       for (uint32_t i = tid; i < nset; i += nthr) {
         const uint32_t p = __ldg(prm.P + i), k = p / 30u;
@@ -824,87 +970,55 @@ sieve_segments_kernel(const SieveParams prm) {
   }
   __syncthreads();
   if (cur_req >= 0 && cur_gaps) flush();
+  if constexpr (kSolo) {
+    // the last segment to be reduced writes the result and leaves the
+    // accumulators and the control words clear for the next run
+    if (prm.solo.nseg > 1) {
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) s_ctr = atomicAdd(&prm.ctl->done, 1u);
+      __syncthreads();
+      if (s_ctr != (uint32_t)prm.solo.nseg - 1u) return;
+      __threadfence();
+    } else {
+      __syncthreads();
+    }
+    // (the segment is done with: its memory serves)
+    finalize_request<true>(prm.solo, 0u, prm.segs, prm.acc, prm.large, &prm.ctl->n_large, prm.large_cap,
+                           &prm.out->res, smem);
+    __syncthreads();
+    if (tid == 0) {
+      prm.out->n_large = __ldcg(&prm.ctl->n_large);
+      prm.ctl->n_large = 0;
+      prm.ctl->done = 0;
+    }
+  }
 }
 
-// One CTA per request: seeds 2, 3, 5, gaps across segment boundaries, the
-// largest gap, and the final counts (the reference's host-side conventions,
-// context.cu:321-322,462-524, restated for a half-open [a, b)).
+__global__ void __launch_bounds__(kMaxThreads, 1) sieve_segments_kernel(const SieveParams prm) {
+  sieve_body<false>(prm);
+}
+
+// A lone request in one launch.  A range of one wave or less leaves most of
+// its time in launches, copies and, at high offsets, in one CTA per segment
+// walking all sieving primes (a 4096-wide window at 10^12: 82 us in one CTA).
+// Here the request comes as a parameter, `slices` CTAs share each segment's
+// units and merge what they cleared in L2, the last of them reduces the
+// segment, and the last segment writes the result to host memory.  No CTA
+// waits for another.
+__global__ void __launch_bounds__(kMaxThreads, 1) solo_kernel(const __grid_constant__ SieveParams prm) {
+  sieve_body<true>(prm);
+}
+
 __global__ void __launch_bounds__(256)
 finalize_kernel(const ReqDesc* __restrict__ reqs, const BatchHdr* __restrict__ hdr,
                 const SegRec* __restrict__ segs, ReqAccum* __restrict__ acc, LargeGapRec* large,
                 unsigned int* n_large, uint32_t large_cap, ReqResult* __restrict__ out) {
-  const uint32_t r = blockIdx.x, tid = threadIdx.x;
+  const uint32_t r = blockIdx.x;
   if (r >= hdr->nreq) return;       // fixed-size launches (graph replay) cover capacity
+  __shared__ __align__(8) uint32_t tmp[kFinalWords];
   const ReqDesc R = reqs[r];
-  ReqAccum* A = acc + r;
-  const SegRec* S = segs + R.seg_base;
-  __shared__ uint64_t s_bg[256], s_bs[256];
-
-  const bool in2 = R.a <= 2 && 2 < R.b, in3 = R.a <= 3 && 3 < R.b, in5 = R.a <= 5 && 5 < R.b;
-  const uint64_t seed_first = in2 ? 2 : in3 ? 3 : in5 ? 5 : 0;
-  const uint64_t seed_last = in5 ? 5 : in3 ? 3 : in2 ? 2 : 0;
-
-  uint64_t bg = 0, bs = 0;
-  auto consider = [&](uint64_t g, uint64_t st) {
-    if (g > bg || (g == bg && g && st < bs)) { bg = g; bs = st; }
-  };
-  if (tid == 0 && (R.rflags & kReqGaps)) {
-    if (in2 && in3) { atomicAdd(&A->hist[0], 1ull); consider(1, 2); }
-    if (in3 && in5) { atomicAdd(&A->hist[1], 1ull); consider(2, 3); }
-  }
-  const bool want_gaps = (R.rflags & kReqGaps) != 0;
-  for (uint64_t i = want_gaps ? tid : R.nseg; i < R.nseg; i += blockDim.x) {
-    const SegRec s = S[i];
-    if (s.max_gap) consider(s.max_gap, s.max_gap_start);
-    if (!s.first) continue;
-    uint64_t prev = 0;
-    for (uint64_t j = i; j-- > 0;) {
-      if (S[j].first) { prev = S[j].last; break; }
-    }
-    if (!prev) prev = seed_last;
-    if (!prev) continue;
-    const uint64_t g = s.first - prev;
-    const uint64_t bin = g >> 1;
-    atomicAdd(&A->hist[bin < (uint64_t)kHistBins ? bin : kHistBins - 1], 1ull);
-    consider(g, prev);
-    if (g >= kLargeGap) {
-      const unsigned idx = atomicAdd(n_large, 1u);
-      if (idx < large_cap) {
-        LargeGapRec lr; lr.pos = s.first; lr.gap = (uint32_t)g; lr.req = r;
-        large[idx] = lr;
-      }
-    }
-  }
-  s_bg[tid] = bg; s_bs[tid] = bs;
-  __syncthreads();
-  for (uint32_t w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (tid < w) {
-      const uint64_t g2 = s_bg[tid + w], t2 = s_bs[tid + w];
-      if (g2 > s_bg[tid] || (g2 == s_bg[tid] && g2 && t2 < s_bs[tid])) { s_bg[tid] = g2; s_bs[tid] = t2; }
-    }
-    __syncthreads();
-  }
-  ReqResult* O = out + r;
-  for (uint32_t b = tid; b < (uint32_t)kHistBins; b += blockDim.x) O->hist[b] = A->hist[b];
-  if (tid == 0) {
-    const uint64_t ns = (uint64_t)in2 + in3 + in5;
-    const uint64_t wc = A->count;
-    O->count = wc + ns;
-    O->c41 = A->c41 + (in5 ? 1 : 0);
-    O->c43 = (wc - A->c41) + (in3 ? 1 : 0);
-    O->c31 = A->c31;
-    O->c32 = (wc - A->c31) + (in2 ? 1 : 0) + (in5 ? 1 : 0);
-    uint64_t f = seed_first, l = seed_last;
-    if (!f) {
-      for (uint64_t i = 0; i < R.nseg; ++i) if (S[i].first) { f = S[i].first; break; }
-    }
-    for (uint64_t i = R.nseg; i-- > 0;) if (S[i].last) { l = S[i].last; break; }
-    O->first = f;
-    O->last = l;
-    O->max_gap = s_bg[0];
-    O->max_gap_start = s_bg[0] ? s_bs[0] : 0;
-    O->num_gaps = O->count ? O->count - 1 : 0;
-  }
+  finalize_request<false>(R, r, segs + R.seg_base, acc + r, large, n_large, large_cap, out + r, tmp);
 }
 
 // Bucket fill: one CTA per work item (a request, a run of its bucket primes
@@ -1164,6 +1278,20 @@ cudaError_t launch_sieve(const SieveParams& prm, uint32_t grid, uint32_t threads
   if (rc) return (cudaError_t)rc;
   if (grid == 0) return cudaSuccess;
   sieve_segments_kernel<<<grid, threads, smem, stream>>>(prm);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_solo(const SieveParams& prm, uint32_t threads, cudaStream_t stream) {
+  const size_t smem = std::max(sieve_smem_bytes(prm.seg_bytes, threads), sizeof(uint32_t) * (size_t)kFinalWords);
+  static AttrCache attr;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const int rc = attr.ensure(dev, smem, [](size_t n) {
+    return (int)cudaFuncSetAttribute(solo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+  });
+  if (rc) return (cudaError_t)rc;
+  solo_kernel<<<(uint32_t)prm.solo.nseg * prm.slices, threads, smem, stream>>>(prm);
   return cudaGetLastError();
 }
 

@@ -209,6 +209,25 @@ struct ReqDesc {
 };
 
 constexpr uint32_t kReqGaps = 1u;
+
+// A request's edge masks: the bits of its first word's first byte that stand for
+// numbers >= a, and those of its last word (of a last segment of nbytes) that
+// stand for numbers < b.
+__host__ __device__ inline uint32_t first_word_mask(const ReqDesc& R) {
+  uint32_t keep = ~0u;
+  for (uint32_t o = 0; o < 8; ++o)
+    if (30ull * R.k_lo + ((kW30Packed >> (8u * o)) & 0xFFu) < R.a) keep &= ~(1u << o);
+  return keep;
+}
+__host__ __device__ inline uint32_t last_word_mask(const ReqDesc& R, uint32_t nbytes) {
+  uint32_t m = 0;
+  for (uint32_t o = 0; o < 8; ++o)
+    if (30ull * (R.k_hi - 1) + ((kW30Packed >> (8u * o)) & 0xFFu) >= R.b) m |= 1u << o;
+  uint32_t keep = ~(m << (((nbytes - 1u) & 3u) << 3));
+  const uint32_t rem = nbytes & 3u;                        // bytes past the end
+  if (rem) keep &= (1u << (rem << 3)) - 1u;
+  return keep;
+}
 // Segments whose bucket lists are filled and held at once: a request of
 // more segments is sieved in windows of this many, the lists of one window
 // reusing the same memory (fill-kernel shared counts, 16-bit packing, and
@@ -259,8 +278,8 @@ struct ReqSpan {
 };
 
 // Per segment: first/last prime (absolute, 0 = none), the largest gap
-// strictly inside the segment and its first prime.
-struct SegRec {
+// strictly inside the segment and its first prime.  Read in 16-byte halves.
+struct alignas(16) SegRec {
   uint64_t first, last;
   uint64_t max_gap_start;
   uint32_t max_gap;
@@ -291,6 +310,21 @@ struct ReqResult {
   uint64_t hist[kHistBins];
 };
 
+// A lone request's result in one piece: what the host reads.
+struct SoloResult {
+  ReqResult res;
+  uint32_t n_large;          // large gaps recorded
+  uint32_t pad;
+};
+
+constexpr uint32_t kSoloMaxSegs = 1024;
+struct SoloCtl {
+  uint32_t seg_done[kSoloMaxSegs];   // slices of each segment that are merged
+  uint32_t done;                     // segments that are reduced
+  uint32_t n_large;
+  uint32_t pad[2];
+};
+
 struct SieveParams {
   const ReqDesc* reqs;
   const BatchHdr* hdr;
@@ -318,6 +352,15 @@ struct SieveParams {
   // a request sits at slot si - list_seg0 (the window's first segment).
   uint64_t item_lo, item_hi;
   uint64_t list_seg0;
+  // The one-launch form (solo_kernel): a lone request without lists whose
+  // segments fit one CTA per SM each, slices CTAs sharing a segment's primes.
+  ReqDesc solo;
+  uint32_t slices;
+  uint32_t low_k;            // wheel byte past every prime that may sieve (rounded to a row)
+  uint32_t keep0, keepl;     // edge masks of the first and the last segment
+  uint32_t* merge;           // slices > 1: words of all segments, all ones between runs
+  SoloCtl* ctl;              // all zero between runs
+  SoloResult* out;           // where the result goes (host memory the device can write)
 };
 
 struct FillParams {
