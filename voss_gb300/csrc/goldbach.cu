@@ -4,7 +4,7 @@
 //    p with n - p prime.  The reference walks the prime list per n and stops
 //    at the first p whose partner is set in a 64-bit-per-64-numbers bitmap
 //    (goldbach_upto.cu:25-46); it keeps only the counterexamples.  Here one
-//    CTA holds 32768 even n as a bit set U of unresolved n; for p = 3, 5, 7...
+//    CTA holds 65536 even n as a bit set U of unresolved n; for p = 3, 5, 7...
 //    the partners n - p of the whole tile are one shifted window of an
 //    odd-number bitmap, so U & window resolves 32 n per word operation.  The
 //    smallest p per n, its maximum and its histogram come out; the
@@ -24,7 +24,6 @@
 #include <new>
 #include <vector>
 
-#include "attr_cache.h"
 #include "goldbach.h"
 #include "voss/voss.h"
 
@@ -90,14 +89,6 @@ constexpr uint32_t kGbList = 256;
 // kGbTile/32 + 1 words past the bitmap).
 constexpr uint64_t kGbPad = kGbTile / 32 + 64;
 
-// Does any of this thread's n wait for a prime?
-__device__ __forceinline__ bool any_open(const uint32_t (&U)[kGbWords]) {
-  uint32_t x = 0;
-#pragma unroll
-  for (int q = 0; q < kGbWords; ++q) x |= U[q];
-  return x != 0;
-}
-
 struct GbOut {
   uint32_t* minp;                    // optional, index (n-4)/2
   unsigned long long* hist;          // by p
@@ -110,7 +101,12 @@ struct GbOut {
   unsigned int* err;                 // 1: the prime list ran out before n/2
 };
 
-__global__ void __launch_bounds__(kGbThreads, 4)
+// kMinp: write the smallest p of every n (out.minp).  Six blocks per SM (40
+// registers) hide the sparse phase of one behind the walk of the others: 0.76
+// ms at N = 10^9 for the whole plan against 0.82 with four; 1.64 before the
+// window words stayed in registers and the blocks summed their totals.
+template <bool kMinp>
+__global__ void __launch_bounds__(kGbThreads, 6)
 goldbach_minp_kernel(const uint32_t* __restrict__ odd,
                      const uint32_t* __restrict__ oddp, uint32_t noddp, uint64_t N,
                      uint64_t ntiles, GbOut out) {
@@ -120,7 +116,7 @@ goldbach_minp_kernel(const uint32_t* __restrict__ odd,
   __shared__ uint32_t s_open[3], s_cnt;
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
   const uint64_t n_last = N & ~1ull;           // largest even n
-  uint32_t lmax = 0;
+  uint32_t lmax = 0;                           // of p >= kGbSmemHist (the others: from the histogram)
   uint32_t chk = 0;                            // checks so far (the same in every thread)
   unsigned long long lsum = 0, lprobes = 0;
   for (uint32_t i = tid; i < kGbSmemHist; i += kGbThreads) shist[i] = 0;
@@ -141,10 +137,27 @@ goldbach_minp_kernel(const uint32_t* __restrict__ odd,
     bool exhausted = true;
     bool sparse = false;
     uint32_t pi = 0;
+    uint32_t probes = 0;
+    // Bit j of this thread's word q is n = n0 + 2*(32*(kGbWords*tid + q) + j); its
+    // partner n - p is odd bit m - h + 32*(kGbWords*tid + q) + j with m = n0 / 2
+    // and h = (p + 1) / 2, so the thread's windows are consecutive bitmap words
+    // shifted by (m - h) mod 32.  They stay in registers: m - h moves on by one
+    // word per 64 of p (five times over the first 60 primes).  Loaded for each
+    // prime, at a lane stride of kGbWords words, they took 72 L1 wavefronts
+    // per warp and prime and 0.8 of the kernel's 1.4 ms at N = 10^9; now issue
+    // bounds the walk.
+    uint32_t a[kGbWords + 1];
+    const uint64_t m = n0 >> 1;
+    const uint32_t* const wp0 = odd + ((m >> 5) + kGbWords * tid);
+    const int32_t mr = (int32_t)(m & 31u);
+    const uint32_t plim = (uint32_t)umin64(nmax >> 1, 0xFFFFFFFFull);       // 2p <= nmax
+    int32_t cur = 1;                           // the word loaded (never positive)
+    uint32_t pnext = __ldg(oddp);
     if (tid == 0) s_cnt = 0;                   // list of the sparse phase (ordered by the first check's barrier)
     for (; pi < noddp; ++pi) {
-      const uint32_t p = __ldg(oddp + pi);
-      if (2ull * p > nmax) { exhausted = false; break; }
+      const uint32_t p = __reduce_max_sync(0xFFFFFFFFu, pnext);     // warp-uniform to the compiler
+      pnext = __ldg(oddp + min(pi + 1u, noddp - 1u));
+      if (p > plim) { exhausted = false; break; }
       if ((pi & 7u) == 0) {
         // the tile's open n, summed over the block into one of three
         // counters taken in turn over all checks of all tiles (the next one
@@ -158,47 +171,48 @@ goldbach_minp_kernel(const uint32_t* __restrict__ odd,
         if (lane == 0 && mine) atomicAdd(&s_open[r], mine);
         if (tid == 0) s_open[(r + 1u) % 3u] = 0;
         __syncthreads();
-        const uint32_t open = s_open[r];
+        const uint32_t open = __reduce_max_sync(0xFFFFFFFFu, s_open[r]);
         if (open == 0) { exhausted = false; break; }
         if (open <= kGbList) { sparse = true; break; }
       }
-      // bit j of this thread's word q is n = n0 + 2*(32*(4*tid + q) + j); its
-      // partner n - p is odd bit base + 32*(4*tid + q) + j, so the thread's
-      // four windows are five consecutive bitmap words shifted by base mod 32
-      const int64_t base = ((int64_t)n0 - (int64_t)p - 1) / 2;   // exact: n0 even, p odd
+      const int32_t bit = mr - (int32_t)((p + 1u) >> 1);
+      const int32_t word = bit >> 5;
+      if (word != cur) {
+        const uint32_t* wp = wp0 + word;
+        if (word == cur - 1 && cur <= 0) {
+#pragma unroll
+          for (int q = kGbWords; q > 0; --q) a[q] = a[q - 1];
+          a[0] = __ldg(wp);
+        } else {
+#pragma unroll
+          for (int q = 0; q <= kGbWords; ++q) a[q] = __ldg(wp + q);
+        }
+        cur = word;
+      }
+      const uint32_t sh = (uint32_t)bit & 31u;
       uint32_t nres = 0;
-      if (any_open(U)) {
-        const uint32_t* wp = odd + ((base >> 5) + (int64_t)(kGbWords * tid));
-        const uint32_t sh = (uint32_t)base & 31u;
-        uint32_t a[kGbWords + 1];
 #pragma unroll
-        for (int q = 0; q <= kGbWords; ++q) a[q] = __ldg(wp + q);
-#pragma unroll
-        for (int q = 0; q < kGbWords; ++q) {
-          if (!U[q]) continue;
-          ++lprobes;
-          uint32_t hit = U[q] & __funnelshift_r(a[q], a[q + 1], sh);
-          if (!hit) continue;
-          U[q] &= ~hit;
-          nres += __popc(hit);
-          if (out.minp) {
-            const uint64_t o = obase + 32u * (tid * kGbWords + q);
-            do {
-              const uint32_t j = (uint32_t)__ffs(hit) - 1u;
-              hit &= hit - 1u;
-              out.minp[o + j] = p;
-            } while (hit);
-          }
+      for (int q = 0; q < kGbWords; ++q) {
+        probes += min(U[q], 1u);
+        uint32_t hit = U[q] & __funnelshift_r(a[q], a[q + 1], sh);
+        U[q] &= ~hit;
+        nres += __popc(hit);
+        if (kMinp) {
+          const uint64_t o = obase + 32u * (tid * kGbWords + q);
+          for (; hit; hit &= hit - 1u) out.minp[o + (uint32_t)__ffs(hit) - 1u] = p;
         }
       }
       // the n resolved at p, per warp: one histogram update
-      if (nres) { lmax = max(lmax, p); lsum += (unsigned long long)p * nres; }
       const uint32_t wres = __reduce_add_sync(0xFFFFFFFFu, nres);
-      if (lane == 0 && wres) {
-        if (p < kGbSmemHist) atomicAdd(&shist[p], wres);
-        else atomicAdd(&out.hist[p], (unsigned long long)wres);
+      if (p < kGbSmemHist) {
+        if (lane == 0) atomicAdd(&shist[p], wres);
+      } else if (lane == 0 && wres) {
+        atomicAdd(&out.hist[p], (unsigned long long)wres);
+        lmax = max(lmax, p);
+        lsum += (unsigned long long)p * wres;
       }
     }
+    lprobes += probes;
     if (sparse) {
       // Few n are left open: gather them into a shared list, then eight
       // lanes per n test eight primes at a time (from the first prime not
@@ -244,11 +258,14 @@ goldbach_minp_kernel(const uint32_t* __restrict__ odd,
           bool done = true;
           if (hit) {
             if (sl == 0) {
-              if (out.minp) out.minp[obase + t] = pm;
-              lmax = max(lmax, pm);
-              lsum += pm;
-              if (pm < kGbSmemHist) atomicAdd(&shist[pm], 1u);
-              else atomicAdd(&out.hist[pm], 1ull);
+              if (kMinp) out.minp[obase + t] = pm;
+              if (pm < kGbSmemHist) {
+                atomicAdd(&shist[pm], 1u);
+              } else {
+                atomicAdd(&out.hist[pm], 1ull);
+                lmax = max(lmax, pm);
+                lsum += pm;
+              }
             }
           } else if (oob | ool) {
             if (sl == 0) {
@@ -291,12 +308,35 @@ goldbach_minp_kernel(const uint32_t* __restrict__ odd,
     }
   }
   __syncthreads();
-  for (uint32_t i = tid; i < kGbSmemHist; i += kGbThreads)
-    if (shist[i]) atomicAdd(&out.hist[i], (unsigned long long)shist[i]);
+  for (uint32_t i = tid; i < kGbSmemHist; i += kGbThreads) {
+    const uint32_t c = shist[i];
+    if (!c) continue;
+    atomicAdd(&out.hist[i], (unsigned long long)c);
+    lmax = max(lmax, i);
+    lsum += (unsigned long long)i * c;
+  }
+  // one addition per block: additions of all threads to one address took
+  // 130 us at every N from 10^8 on (608 blocks)
   lmax = __reduce_max_sync(0xFFFFFFFFu, lmax);
-  if (lane == 0) atomicMax(out.max_minp, lmax);
-  atomicAdd(out.sum_minp, lsum);
-  atomicAdd(out.probes, lprobes);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    lsum += __shfl_down_sync(0xFFFFFFFFu, lsum, d);
+    lprobes += __shfl_down_sync(0xFFFFFFFFu, lprobes, d);
+  }
+  __shared__ unsigned long long s_sum[kGbThreads / 32], s_probes[kGbThreads / 32];
+  __shared__ uint32_t s_max[kGbThreads / 32];
+  if (lane == 0) { s_sum[tid >> 5] = lsum; s_probes[tid >> 5] = lprobes; s_max[tid >> 5] = lmax; }
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < kGbThreads / 32; ++w) {
+      lsum += s_sum[w];
+      lprobes += s_probes[w];
+      lmax = max(lmax, s_max[w]);
+    }
+    atomicMax(out.max_minp, lmax);
+    atomicAdd(out.sum_minp, lsum);
+    atomicAdd(out.probes, lprobes);
+  }
 }
 
 __global__ void sophie_germain_kernel(const uint32_t* __restrict__ wb, uint64_t N,
@@ -441,7 +481,7 @@ static void goldbach_plan_set(GoldbachPlan* g, Engine& E, uint64_t N) {
   g->ce.reserve(8 * g->ce_cap);
   g->ntiles = N >= 6 ? ((N & ~1ull) - 6) / (2ull * kGbTile) + 1 : 0;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, goldbach_minp_kernel, kGbThreads, kGbSmemBytes) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, goldbach_minp_kernel<false>, kGbThreads, kGbSmemBytes) !=
           cudaSuccess || per_sm < 1)
     per_sm = 1;
   g->grid = (uint32_t)std::min<uint64_t>(g->ntiles, (uint64_t)E.sm_count * per_sm);
@@ -525,15 +565,9 @@ void goldbach_plan_launch(GoldbachPlan* g, cudaStream_t s) {
   o.err = reinterpret_cast<unsigned int*>(sc + 4);
   o.ce = g->ce.as<unsigned long long>();
   o.ce_cap = g->ce_cap;
-  static AttrCache attr;          // per device, thread-safe
-  int dev = 0;
-  check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
-  check_cuda((cudaError_t)attr.ensure(dev, kGbSmemBytes, [](size_t n) {
-               return (int)cudaFuncSetAttribute(goldbach_minp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)n);
-             }), "goldbach smem");
-  goldbach_minp_kernel<<<g->grid, kGbThreads, kGbSmemBytes, s>>>(odd, g->oddp.as<uint32_t>(), kGoldbachPrimes,
-                                                                  g->N, g->ntiles, o);
+  static_assert(kGbSmemBytes <= 48u * 1024u, "no shared-memory attribute needed");
+  auto* const kernel = g->want_minp ? goldbach_minp_kernel<true> : goldbach_minp_kernel<false>;
+  kernel<<<g->grid, kGbThreads, kGbSmemBytes, s>>>(odd, g->oddp.as<uint32_t>(), kGoldbachPrimes, g->N, g->ntiles, o);
   check_cuda(cudaGetLastError(), "goldbach_minp_kernel");
 }
 
