@@ -110,8 +110,13 @@ __device__ __forceinline__ void and_word_if(uint32_t a, uint32_t mask, bool on) 
 __device__ __forceinline__ void clear_bit(uint32_t seg, uint32_t v) {
   and_word(seg + 4u * (v >> 5), __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, v));
 }
-__device__ __forceinline__ void clear_bit_below(uint32_t seg, uint32_t v, uint32_t end) {
-  if (v < end) clear_bit(seg, v);
+// (The test is made on the word's address, so up to 31 bits past `end` may be
+// cleared: send is the address past the last word, whose spare bits are masked
+// when it is scanned.)
+__device__ __forceinline__ void clear_bit_below(uint32_t seg, uint32_t v, uint32_t send) {
+  const uint32_t a = seg + 4u * (v >> 5), m = __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, v);
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.u32 p, %0, %2;\n\t@p red.shared.and.b32 [%0], %1;\n\t}"
+               :: "r"(a), "r"(m), "r"(send) : "memory");
 }
 
 // The eight class residues of table prime i (32 bytes, two vector loads).
@@ -662,16 +667,48 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
           uint2 e = __ldg(W + min(i, cend - 1u));
           const uint32_t pfirst = __reduce_min_sync(0xFFFFFFFFu, 30u * e.x + cc);
           uint32_t left = 1u << (wlog - 5u);            // batches of 32 primes
-          if (pfirst >= unb) {
+          const uint32_t wend4 = sseg + ((unb + 3u) & ~3u);       // address past the last word
+          if (pfirst >= 15u * unb) {
+            // at most one hit at all (cofactors coprime to 30 lie 2 apart or
+            // more): the first multiple p (30 a + w) of the segment is found
+            // directly, from 30 (k0 mod p) / p and the next w from there.  (As
+            // the smallest of the eight classes' hits, below, a prime took 40
+            // operations on the integer pipe, twice its share; here 16.)
+            constexpr uint32_t kCoprime = 0xA08A2882u;    // residues 1 7 11 13 17 19 23 29, and 31 for the next turn's 1
+            auto mark = [&](uint2 q) {
+              const uint32_t p = 30u * q.x + cc, inv = q.y;
+              uint32_t m = k0l - __umulhi(k0s, inv) * p;
+              m = min(m, m - p);
+              m = min(m, m - p);
+              const uint32_t m30 = 30u * m;
+              uint32_t r = __umulhi(m30, inv) >> 10;      // 30 m / p, or one less
+              r += m30 - r * p >= p ? 2u : 1u;            // cofactors from r on give numbers >= 30 k0
+              const uint32_t w = r + (uint32_t)__ffs(kCoprime >> r) - 1u;
+              const uint32_t n = w * p - m30;             // the hit's number in the segment, at most 6 p
+              const uint32_t byte = __umulhi(n, 143165577u);            // n / 30 (exact below 3 * 10^8)
+              clear_bit_below(sseg, 8u * byte + (((n - 30u * byte) * 17477u) >> 16), wend4);   // W30[o] * 4 / 15 = o
+            };
+            // (So few operations per prime leave the table's L2 reads to bound
+            // the loop at 6 TB/s over the chip; more batches in flight per
+            // warp than one ahead gain nothing.)
+            for (;;) {
+              const uint2 now = e;
+              if (--left) e = __ldg(W + min(i += 32u, cend - 1u));
+              mark(now);
+              if (!left) break;
+            }
+          } else if (pfirst >= unb) {
             // at most one hit per class: positions as bit indices 8 * byte +
             // class, whose low bits also give the mask
             uint32_t step[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) step[j] = C.bstep[j];
-            // from 2.5 segments on, cofactors w_j and w_(j+4) lie 12/30 to
-            // 18/30 of p apart, so at most one of the two hits is inside
-            const bool sparse = 2u * pfirst >= 5u * unb;
-            const uint32_t end = 8u * unb;
+            // Hits of cofactors w and w' (mod 30) lie at least |w - w'| / 30 and
+            // 1 - |w - w'| / 30 of p apart, so of a group of classes whose
+            // cofactors keep a distance of 12 or 6 round the circle at most one
+            // hit is inside, from 2.5 or 5 segments on: one clear for the
+            // smallest of the group.
+            const uint32_t group = pfirst >= 5u * unb ? 4u : 2u * pfirst >= 5u * unb ? 2u : 1u;
             for (;;) {
               const uint32_t p = 30u * e.x + cc;
               uint32_t m = k0l - __umulhi(k0s, e.y) * p;
@@ -689,12 +726,15 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
                 y += (j == 1 || j == 7 ? t6 : j == 3 || j == 5 ? t2 : t4) + step[j];
                 v[j] = min(y, y + p8);
               }
-              if (sparse) {
+              if (group == 4u) {                   // w = 1 7 13 19 and 11 17 23 29
+                clear_bit_below(sseg, min(min(v[0], v[1]), min(v[3], v[5])), wend4);
+                clear_bit_below(sseg, min(min(v[2], v[4]), min(v[6], v[7])), wend4);
+              } else if (group == 2u) {                   // w_j and w_(j+4): 16, 12, 12, 16 apart
 #pragma unroll
-                for (int j = 0; j < 4; ++j) clear_bit_below(sseg, min(v[j], v[j + 4]), end);
+                for (int j = 0; j < 4; ++j) clear_bit_below(sseg, min(v[j], v[j + 4]), wend4);
               } else {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) clear_bit_below(sseg, v[j], end);
+                for (int j = 0; j < 8; ++j) clear_bit_below(sseg, v[j], wend4);
               }
               if (!left) break;
             }
@@ -836,7 +876,8 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
         // the byte histogram (its primes and the gaps inside it follow from
         // that when the request is flushed), the gap into it from the
         // previous prime in the gap histogram, and the largest such gap is
-        // kept as g << 23 | (2^23 - 1 - end), the earliest first on ties.
+        // kept as g << 23 | (2^23 - 1 - end), the earliest first on ties
+        // (nv and npv are 2^23 - 1 - the gap's end and start).
         // (Before, a 16-byte table entry per byte brought the inner gaps as
         // packed counters: 12 shared-memory wavefronts and 35 instructions
         // per byte and warp, now 7 and 24: [9*10^11, 10^12) 16.5 -> 14.8 ms.)
@@ -848,35 +889,37 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
         constexpr uint32_t kWlo = (uint32_t)kW30Packed, kWhi = (uint32_t)(kW30Packed >> 32);
         constexpr uint32_t kEnd = (1u << 23) - 1u;
         static_assert(30u * kMaxSegBytes < kEnd && 2 * kSmemBins < 512, "a gap and its end share 32 bits");
+        const uint32_t tb = (uint32_t)__cvta_generic_to_shared(btab);
         uint32_t fi = wbeg;                         // the run's first prime is its first "previous" one (gap 0)
         while (fi < wend && !seg[fi]) ++fi;
         uint32_t pv = fi < wend ? 120u * fi + word_value(__ffs(seg[fi]) - 1u) : 0u;
         if (fi < wend) first1 = pv + 1u;
-        uint32_t top = 0;
+        uint32_t top = 0, npv = kEnd - pv;
         const uint32_t nsteps = uniform(run);
 #pragma unroll 4
         for (uint32_t i = 0; i < nsteps; ++i) {
           const uint32_t wi = wbeg + i;
           const uint32_t w = wi < wend ? seg[wi] : 0u;
           c41 += __popc(w & m41);
-          const uint32_t vb = 120u * wi;
+          const int nvb = (int)(kEnd - 120u * wi);
 #pragma unroll
           for (uint32_t b = 0; b < 4; ++b) {
             const uint32_t x = (w >> (8u * b)) & 0xFFu;
             if (x) {
-              const uint32_t e = btab[x];
+              uint32_t e;
+              asm volatile("ld.shared.u8 %0, [%1];" : "=r"(e) : "r"(tb + x));
               count_one(bb + 4u * x);
-              const uint32_t r = __byte_perm(kWlo, kWhi, e);      // W30 of the lowest, the highest bit
-              const uint32_t v = vb + 30u * b + (r & 0xFFu);
-              const uint32_t g = min(v - pv, 2u * (uint32_t)kSmemBins);
-              pv = vb + 30u * b + ((r >> 8) & 0xFFu);
+              const int r = (int)__byte_perm(kWlo, kWhi, e);      // bytes: W30 of the lowest, of the highest bit
+              const uint32_t nv = (uint32_t)__dp4a(r, 0x000000FF, nvb - 30 * (int)b);
+              const uint32_t g = min(npv - nv, 2u * (uint32_t)kSmemBins);
+              npv = (uint32_t)__dp4a(r, 0x0000FF00, nvb - 30 * (int)b);
               count_one(hb + 2u * g);
-              top = max(top, (g << 23) + (kEnd - v));
+              top = max(top, g * (1u << 23) + nv);
             }
           }
         }
         if (first1) {
-          last1 = pv + 1u;
+          last1 = kEnd - npv + 1u;
           maxg = top >> 23;
           maxgs = kEnd - (top & kEnd) - maxg;
         }

@@ -233,7 +233,9 @@ __host__ __device__ inline uint32_t last_word_mask(const ReqDesc& R, uint32_t nb
 // reusing the same memory (fill-kernel shared counts, 16-bit packing, and
 // window offsets below 2^30 bytes).
 constexpr uint32_t kMaxBucketSegs = 4096;
-constexpr uint32_t kWheelUnitLog2Max = 8;    // wheel-tier primes per work unit: 2^5 .. 2^8
+// Wheel-tier primes per work unit: 2^5 .. 2^10 ([10^14, 10^14+10^10) without
+// lists: 3.32 / 3.11 ms with at most 2^8 / 2^10).
+constexpr uint32_t kWheelUnitLog2Max = 10;
 constexpr uint32_t kBucketUnit = 1024;       // list entries per work unit of the sieve kernel
 constexpr uint32_t kFillPrimes = 256;        // bucket primes per fill work item
 constexpr uint32_t kFillHits = 16384;        // list entries per fill work item, about
