@@ -41,3 +41,17 @@ def test_kept_buffers_in_any_order(vg, oracle_lib):
         P.set_config(**base)
     sophie(30, 6)
     goldbach(6)
+
+
+@pytest.mark.parametrize("a,b", [(2, 2), (2, 7), (0, 29), (7, 31), (10**6 - 17, 10**6 + 1), (10**12, 10**12 + 3),
+                                 (10**9, 10**9 + 30 * 4 * 4096 - 1), (10**9, 10**9 + 30 * 4 * 4096),
+                                 (10**11 + 1, 10**11 + 30 * 4 * 4096 * 3 + 7), (0, 10**6), (10**13 - 5, 10**13 + 10**6)])
+def test_lists_at_block_edges(vg, oracle_lib, a, b):
+    # one extraction block holds 4096 words of 120 integers
+    want = oracle_lib.primes_in_range(a, b).tolist()
+    assert vg.primes.in_range(a, b) == want
+    if want:
+        assert vg.primes.in_range_with_limit(a, b, len(want)) == want
+        if len(want) > 1:
+            with pytest.raises(vg.VossError):
+                vg.primes.in_range_with_limit(a, b, len(want) - 1)

@@ -819,18 +819,19 @@ constexpr uint32_t kSoloSlicePrimes = 256;
 constexpr uint32_t kSoloListPrimes = 100000;
 constexpr uint32_t kSoloLargeCap = 1u << 14;
 
-const ReqResult* Engine::run_solo(uint64_t a, uint64_t b, std::vector<LargeGapRec>* lg, bool gaps) {
-  if (b <= a || b > kMaxB) return nullptr;
+bool Engine::solo_start(uint64_t a, uint64_t b, bool gaps, uint32_t* bitmap) {
+  if (b <= a || b > kMaxB) return false;
   ensure_table(isqrt_u64(b - 1));
   const Config c = tuned_for(a, b, false);
   const ReqDesc r = describe(a, b, gaps ? kReqGaps : 0u, c);
   const uint64_t ctas = std::min<uint64_t>((uint64_t)sm_count * cfg.ctas_per_sm, kSoloMaxSegs);
-  if (r.nseg > ctas) return nullptr;
+  if (r.nseg > ctas) return false;
   uint64_t slices = 1;
   if (r.nseg * r.seg_bytes <= kSoloMergeBytes)
     slices = std::max<uint64_t>(1, std::min<uint64_t>(ctas / r.nseg, r.nprimes / kSoloSlicePrimes));
+  // (runs with a bitmap never take lists)
   const BucketPlan bp = bucket_plan(c, b, r.nprimes, r.nseg, r.seg_bytes);
-  if (bp.cap && (!cfg.auto_tune || (r.nprimes - bp.bucket_idx) / slices > kSoloListPrimes)) return nullptr;
+  if (bp.cap && !bitmap && (!cfg.auto_tune || (r.nprimes - bp.bucket_idx) / slices > kSoloListPrimes)) return false;
 
   if (!solo.clean) {
     solo.ctl.reserve(sizeof(SoloCtl));
@@ -859,11 +860,22 @@ const ReqResult* Engine::run_solo(uint64_t a, uint64_t b, std::vector<LargeGapRe
   prm.merge = solo.merge.as<uint32_t>();
   prm.ctl = solo.ctl.as<SoloCtl>();
   prm.out = static_cast<SoloResult*>(solo.out.ptr);
+  prm.flags = bitmap ? kFlagBitmap : 0u;
+  prm.bitmap = bitmap;
   solo.clean = false;                        // until the run has ended well
   check_cuda(launch_solo(prm, cfg.threads, stream), "solo_kernel");
-  check_cuda(cudaStreamSynchronize(stream), "sieve run");
+  return true;
+}
+
+const SoloResult* Engine::solo_done() {
   solo.clean = true;
-  const SoloResult* out = static_cast<const SoloResult*>(solo.out.ptr);
+  return static_cast<const SoloResult*>(solo.out.ptr);
+}
+
+const ReqResult* Engine::run_solo(uint64_t a, uint64_t b, std::vector<LargeGapRec>* lg, bool gaps) {
+  if (!solo_start(a, b, gaps, nullptr)) return nullptr;
+  check_cuda(cudaStreamSynchronize(stream), "sieve run");
+  const SoloResult* out = solo_done();
   if (lg) {
     if (out->n_large > kSoloLargeCap)
       throw Error(VOSS_ERR_INTERNAL, "large-gap buffer overflow (" + std::to_string(out->n_large) + " gaps)");

@@ -274,6 +274,13 @@ class Engine {
   // Kernel parameters with the tables filled in.
   SieveParams table_params() const;
 
+  // Enqueue a lone range in one launch on the engine stream, with its wheel
+  // bitmap if `bitmap` has room for it (4-byte words from byte a / 30); false
+  // where that form does not fit the range.  Once the stream has been
+  // synchronised without an error, solo_done() gives the result.
+  bool solo_start(uint64_t a, uint64_t b, bool gaps, uint32_t* bitmap);
+  const SoloResult* solo_done();
+
   // Run ranges synchronously on the engine stream.  share: overlapping
   // ranges sieve their common integers once (not with large-gap output).
   const ReqResult* run(uint32_t n, const uint64_t* a, const uint64_t* b,
@@ -284,7 +291,6 @@ class Engine {
   Engine() = default;
   void init();
   void build_tiles();
-  // A lone range in one launch, or null where that form does not fit it.
   const ReqResult* run_solo(uint64_t a, uint64_t b, std::vector<LargeGapRec>* large, bool gaps);
 };
 

@@ -357,6 +357,10 @@ __global__ void sophie_germain_kernel(const uint32_t* __restrict__ wb, uint64_t 
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
 }
 
+// Widest range tried in one launch (one wave of the largest segments is 1.02 *
+// 10^9 on 152 SMs; the launch itself refuses what does not fit).
+constexpr uint64_t kSoloBitmapWidth = 1ull << 31;
+
 constexpr int kExThreads = 512;
 constexpr int kExWords = 8;
 constexpr uint32_t kExBlockWords = kExThreads * kExWords;
@@ -379,10 +383,23 @@ __global__ void extract_count_kernel(const uint32_t* __restrict__ wb, uint64_t n
   }
 }
 
+// block_offsets: where each block's primes go; null: after those of the blocks
+// before it, whose counts it adds up itself (few blocks, no wait for the host).
 __global__ void extract_write_kernel(const uint32_t* __restrict__ wb, uint64_t nwords,
                                      uint64_t k_lo, const uint64_t* __restrict__ block_offsets,
-                                     uint64_t* __restrict__ out) {
+                                     const uint32_t* __restrict__ block_counts, uint64_t* __restrict__ out) {
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t before = 0;
+  if (!block_offsets) {
+    for (uint32_t i = tid; i < blockIdx.x; i += kExThreads) before += block_counts[i];
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    __shared__ uint32_t sb[kExThreads / 32];
+    if (lane == 0) sb[warp] = before;
+    __syncthreads();
+    before = 0;
+#pragma unroll
+    for (int w = 0; w < kExThreads / 32; ++w) before += sb[w];
+  }
   const uint64_t w0 = blockIdx.x * (uint64_t)kExBlockWords + tid * (uint64_t)kExWords;
   uint32_t words[kExWords];
   uint32_t c = 0;
@@ -412,7 +429,7 @@ __global__ void extract_write_kernel(const uint32_t* __restrict__ wb, uint64_t n
     if (lane < kExThreads / 32) s[lane] = iv - v;
   }
   __syncthreads();
-  uint64_t pos = block_offsets[blockIdx.x] + s[warp] + (incl - c);
+  uint64_t pos = (block_offsets ? block_offsets[blockIdx.x] : before) + s[warp] + (incl - c);
 #pragma unroll
   for (int i = 0; i < kExWords; ++i) {
     uint32_t w = words[i];
@@ -425,15 +442,23 @@ __global__ void extract_write_kernel(const uint32_t* __restrict__ wb, uint64_t n
   }
 }
 
-// Sieve [0, limit] (or [a, b]) into a wheel bitmap on the device.
-const uint32_t* sieve_bitmap(Engine& E, Plan& plan, uint64_t a, uint64_t b_excl, uint64_t* nwords) {
+// Sieve [a, b) into a wheel bitmap on the device, on the engine's stream: in one
+// launch where that fits (*solo, then E.solo_done() has the count), else by the plan.
+const uint32_t* sieve_bitmap(Engine& E, Plan& plan, uint64_t a, uint64_t b_excl, uint64_t* nwords, bool* solo) {
   plan.eng = &E;
   plan.device = E.device;
   plan.timed = false;
-  const uint32_t count_only = 0;          // the readers need no gap scan
-  plan.load(1, &a, &b_excl, kFlagBitmap, &count_only);
-  plan.launch(E.stream);
-  *nwords = (plan.host_reqs[0].k_hi - plan.host_reqs[0].k_lo + 3) / 4;
+  *nwords = ((b_excl + 29) / 30 - a / 30 + 3) / 4;
+  *solo = false;
+  if (b_excl - a <= kSoloBitmapWidth) {
+    plan.bitmap.reserve_ahead((*nwords + 1) * 4);
+    *solo = E.solo_start(a, b_excl, false, plan.bitmap.as<uint32_t>());
+  }
+  if (!*solo) {
+    const uint32_t count_only = 0;          // the readers need no gap scan
+    plan.load(1, &a, &b_excl, kFlagBitmap, &count_only);
+    plan.launch(E.stream);
+  }
   return plan.bitmap.as<uint32_t>();
 }
 
@@ -458,6 +483,8 @@ struct GoldbachPlan {
   uint64_t odd_words = 0, ntiles = 0, ce_cap = 0;
   uint32_t grid = 0;
   bool want_minp = false;
+  bool kept = false;             // the engine's own, used under its lock and on its stream
+  bool solo = false;             // the last launch sieved in one launch
 };
 
 // Size g for N, keeping what it holds.
@@ -505,6 +532,7 @@ constexpr size_t kKeepBytes = 256u << 20;
 struct BitmapWork {
   Plan sieve;                    // in_range, Sophie Germain
   DevBuf counts, offsets, primes, total;
+  HostPinned listed;             // short lists, written by the kernel
   GoldbachPlan gb;
   size_t bytes() const {
     return sieve.bitmap.bytes + counts.bytes + offsets.bytes + primes.bytes + gb.sieve.bitmap.bytes +
@@ -538,8 +566,13 @@ void goldbach_plan_launch(GoldbachPlan* g, cudaStream_t s) {
   {
     uint64_t a = 0, b = g->N + 1;
     const uint32_t count_only = 0;
-    if (!g->sieve.nreq || g->sieve.host_reqs[0].b != b) g->sieve.load(1, &a, &b, kFlagBitmap, &count_only);
-    g->sieve.launch(s);
+    if (g->kept) {
+      uint64_t nw = 0;
+      sieve_bitmap(E, g->sieve, a, b, &nw, &g->solo);
+    } else {
+      if (!g->sieve.nreq || g->sieve.host_reqs[0].b != b) g->sieve.load(1, &a, &b, kFlagBitmap, &count_only);
+      g->sieve.launch(s);
+    }
   }
   const uint32_t* wb = g->sieve.bitmap.as<uint32_t>();
   uint32_t* odd = g->odd.as<uint32_t>() + kGbPad;
@@ -608,6 +641,7 @@ GoldbachResult goldbach_run(Engine& E, uint64_t N, uint32_t* minp_host, uint64_t
   KeptWork work(E);
   GoldbachPlan* const g = &work->gb;
   goldbach_plan_set(g, E, N);
+  g->kept = true;
   const uint64_t nn = (N - 4) / 2 + 1;
   g->want_minp = minp_host != nullptr;
   if (minp_host) g->minp.reserve_ahead(4 * nn);
@@ -623,6 +657,7 @@ GoldbachResult goldbach_run(Engine& E, uint64_t N, uint32_t* minp_host, uint64_t
   if (kernel_ms) check_cuda(cudaEventRecord(e1, E.stream), "event");
   GoldbachResult r;
   goldbach_plan_fetch(g, &r, E.stream);
+  if (g->solo) E.solo_done();
   if (kernel_ms) {
     check_cuda(cudaEventElapsedTime(kernel_ms, e0, e1), "event");
     cudaEventDestroy(e0);
@@ -641,7 +676,8 @@ uint64_t sophie_germain_count(Engine& E, uint64_t N) {
   if (N < 11) return seeds;
   KeptWork work(E);
   uint64_t nw = 0;
-  const uint32_t* wb = sieve_bitmap(E, work->sieve, 0, 2 * N + 2, &nw);
+  bool solo = false;
+  const uint32_t* wb = sieve_bitmap(E, work->sieve, 0, 2 * N + 2, &nw, &solo);
   DevBuf& cnt = work->total;
   cnt.reserve(8);
   check_cuda(cudaMemsetAsync(cnt.ptr, 0, 8, E.stream), "memset");
@@ -650,6 +686,7 @@ uint64_t sophie_germain_count(Engine& E, uint64_t N) {
   unsigned long long c = 0;
   check_cuda(cudaMemcpyAsync(&c, cnt.ptr, 8, cudaMemcpyDeviceToHost, E.stream), "count");
   check_cuda(cudaStreamSynchronize(E.stream), "sophie germain");
+  if (solo) E.solo_done();
   return seeds + c;
 }
 
@@ -657,6 +694,8 @@ uint64_t sophie_germain_count(Engine& E, uint64_t N) {
 // their bitmap, unless they surely hold more than max_count primes; others are
 // counted first, so that an oversized request fails before any bitmap is built.
 constexpr uint64_t kOnePassWidth = 1ull << 31;
+constexpr uint64_t kExMaxOnePass = 1024;       // blocks whose offsets the blocks add up themselves (5 * 10^8 wide)
+constexpr uint64_t kExHostRoom = 65536;        // primes of a list that the kernel writes to host memory
 
 PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count) {
   PrimeList out;
@@ -681,9 +720,32 @@ PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count)
   }
   KeptWork work(E);
   uint64_t nw = 0;
-  const uint32_t* wb = sieve_bitmap(E, work->sieve, a, b + 1, &nw);
+  bool solo = false;
+  const uint32_t* wb = sieve_bitmap(E, work->sieve, a, b + 1, &nw, &solo);
   const uint64_t nblocks = (nw + kExBlockWords - 1) / kExBlockWords;
   work->counts.reserve_ahead(4 * std::max<uint64_t>(nblocks, 1));
+  if (solo && nblocks <= kExMaxOnePass) {
+    // no wait between count and list: the room is what w integers can hold at
+    // most (2 w / ln w primes), a short list goes straight to host memory
+    const double w = (double)(bb - aa) + 2.0;
+    const uint64_t room = std::min<uint64_t>(32 * nw, (uint64_t)(2.0 * w / std::log(w)) + 64);
+    const bool here = room <= kExHostRoom;
+    if (here) work->listed.reserve(8 * kExHostRoom);
+    else work->primes.reserve_ahead(8 * room);
+    uint64_t* const dst = here ? static_cast<uint64_t*>(work->listed.ptr) : work->primes.as<uint64_t>();
+    extract_count_kernel<<<(unsigned)nblocks, kExThreads, 0, E.stream>>>(wb, nw, work->counts.as<uint32_t>());
+    check_cuda(cudaGetLastError(), "extract_count_kernel");
+    extract_write_kernel<<<(unsigned)nblocks, kExThreads, 0, E.stream>>>(wb, nw, a / 30, nullptr,
+                                                                           work->counts.as<uint32_t>(), dst);
+    check_cuda(cudaGetLastError(), "extract_write_kernel");
+    check_cuda(cudaStreamSynchronize(E.stream), "in_range");
+    total = E.solo_done()->res.count;
+    if (!listed() || total == seeds.size()) return out;
+    const uint64_t t = total - seeds.size();
+    if (here) std::memcpy(out.p + seeds.size(), dst, 8 * t);
+    else check_cuda(cudaMemcpy(out.p + seeds.size(), dst, 8 * t, cudaMemcpyDeviceToHost), "primes");
+    return out;
+  }
   work->offsets.reserve_ahead(8 * std::max<uint64_t>(nblocks, 1));
   std::vector<uint32_t> counts(nblocks);
   if (nblocks) {
@@ -693,6 +755,7 @@ PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count)
                "counts");
   }
   check_cuda(cudaStreamSynchronize(E.stream), "counts");
+  if (solo) E.solo_done();
   std::vector<uint64_t> offs(nblocks);
   uint64_t t = 0;
   for (uint64_t i = 0; i < nblocks; ++i) { offs[i] = t; t += counts[i]; }
@@ -702,7 +765,7 @@ PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count)
              "offsets");
   work->primes.reserve_ahead(8 * t);
   extract_write_kernel<<<(unsigned)nblocks, kExThreads, 0, E.stream>>>(
-      wb, nw, work->sieve.host_reqs[0].k_lo, work->offsets.as<uint64_t>(), work->primes.as<uint64_t>());
+      wb, nw, a / 30, work->offsets.as<uint64_t>(), nullptr, work->primes.as<uint64_t>());
   check_cuda(cudaGetLastError(), "extract_write_kernel");
   check_cuda(cudaMemcpyAsync(out.p + seeds.size(), work->primes.ptr, 8 * t, cudaMemcpyDeviceToHost, E.stream),
              "primes");

@@ -315,8 +315,10 @@ __device__ __forceinline__ void finalize_request(const ReqDesc& R, uint32_t r, c
   const uint64_t seed_first = in2 ? 2 : in3 ? 3 : in5 ? 5 : 0;
   const uint64_t seed_last = in5 ? 5 : in3 ? 3 : in2 ? 2 : 0;
   const bool gaps = (R.rflags & kReqGaps) != 0;
+  // the accumulators of other CTAs, loaded while the records are folded
   uint64_t wc = 0, a41 = 0, a31 = 0;
   if (tid == 0) { wc = __ldcg(&A->count); a41 = __ldcg(&A->c41); a31 = __ldcg(&A->c31); }
+  const uint64_t h0 = tid < (uint32_t)kHistBins ? __ldcg(&A->hist[tid]) : 0;
   for (uint32_t b = tid; b < (uint32_t)kHistBins; b += blockDim.x) joins[b] = 0;
   __syncthreads();
 
@@ -359,20 +361,23 @@ __device__ __forceinline__ void finalize_request(const ReqDesc& R, uint32_t r, c
     first = f2 < first ? f2 : first;
     last = l2 > last ? l2 : last;
   };
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    const uint64_t g2 = __shfl_down_sync(0xFFFFFFFFu, bg, d), s2 = __shfl_down_sync(0xFFFFFFFFu, bs, d);
-    const uint64_t f2 = __shfl_down_sync(0xFFFFFFFFu, first, d), l2 = __shfl_down_sync(0xFFFFFFFFu, last, d);
-    fold(g2, s2, f2, l2);
+  const uint32_t warps = (uint32_t)min((uint64_t)(blockDim.x >> 5), (R.nseg + 31u) / 32u);   // those with records
+  if (warp < max(warps, 1u)) {
+#pragma unroll 1
+    for (int d = 16; d > 0; d >>= 1) {
+      const uint64_t g2 = __shfl_down_sync(0xFFFFFFFFu, bg, d), s2 = __shfl_down_sync(0xFFFFFFFFu, bs, d);
+      const uint64_t f2 = __shfl_down_sync(0xFFFFFFFFu, first, d), l2 = __shfl_down_sync(0xFFFFFFFFu, last, d);
+      fold(g2, s2, f2, l2);
+    }
+    if (lane == 0) { part[4 * warp] = bg; part[4 * warp + 1] = bs; part[4 * warp + 2] = first; part[4 * warp + 3] = last; }
   }
-  if (lane == 0) { part[4 * warp] = bg; part[4 * warp + 1] = bs; part[4 * warp + 2] = first; part[4 * warp + 3] = last; }
   __syncthreads();
   for (uint32_t b = tid; b < (uint32_t)kHistBins; b += blockDim.x) {
-    O->hist[b] = __ldcg(&A->hist[b]) + joins[b];
+    O->hist[b] = (b == tid ? h0 : __ldcg(&A->hist[b])) + joins[b];
     if (kClean) A->hist[b] = 0;
   }
   if (tid == 0) {
-    for (uint32_t w = 1; w < blockDim.x >> 5; ++w) fold(part[4 * w], part[4 * w + 1], part[4 * w + 2], part[4 * w + 3]);
+    for (uint32_t w = 1; w < warps; ++w) fold(part[4 * w], part[4 * w + 1], part[4 * w + 2], part[4 * w + 3]);
     const uint64_t ns = (uint64_t)in2 + in3 + in5;
     const uint64_t count = wc + ns;
     O->count = count;
@@ -859,7 +864,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       if (wbeg < wend && wend == nwords) seg[nwords - 1u] &= S.keepl;
       if (prm.flags & kFlagBitmap) {
         __syncthreads();
-        uint32_t* dst = prm.bitmap + ((k0 - prm.reqs[0].k_lo) >> 2);
+        uint32_t* dst = prm.bitmap + ((k0 - (kSolo ? prm.solo.k_lo : prm.reqs[0].k_lo)) >> 2);
         for (uint32_t w = tid; w < nwords; w += nthr) dst[w] = seg[w];
       }
       GapSink sk;
