@@ -204,7 +204,7 @@ __device__ __forceinline__ void count_one(uint32_t a) {
 // live in wheel byte 0, 31 in byte 1), 1, and the request's ends.
 struct SegItem {
   uint64_t item, k0, bbase;
-  uint32_t req, nbytes, np, split, wheel, rflags, bcnt, valid;
+  uint32_t req, nbytes, np, split, wheel, rflags, bcnt, valid, mix;
   uint32_t and0, or0, keep0, keepl;
 };
 
@@ -274,6 +274,7 @@ __device__ __noinline__ void claim_item(unsigned long long* queue, const ReqDesc
     }
     d.item = item; d.valid = 1;
     d.req = r; d.k0 = k0; d.nbytes = nb; d.np = a;
+    d.mix = a && P[a - 1u] >= 2u * nb;
     set_item(d, R, si == 0 ? first_word_mask(R) : ~0u, k0 + nb == R.k_hi ? last_word_mask(R, nb) : ~0u);
   }
 }
@@ -470,7 +471,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       const uint32_t si = blockIdx.x / slices;
       d.k0 = R.k_lo + (uint64_t)si * R.seg_bytes;
       d.nbytes = (uint32_t)min((uint64_t)R.seg_bytes, R.k_hi - d.k0);
-      d.item = si; d.valid = 1; d.req = 0; d.np = R.nprimes; d.bcnt = 0; d.bbase = 0;
+      d.item = si; d.valid = 1; d.req = 0; d.np = R.nprimes; d.bcnt = 0; d.bbase = 0; d.mix = 0;
       set_item(d, R, si == 0 ? prm.keep0 : ~0u, si + 1u == (uint32_t)R.nseg ? prm.keepl : ~0u);
       s_item[1].valid = 0;
     }
@@ -584,6 +585,12 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
         claim_item(prm.queue, prm.reqs, prm.P, prm.bcount, prm.item_lo, item_end, prm.list_seg0, nreq,
                    s_item[cur ^ 1u], lane);
       const uint32_t nunits = nscan + (bcnt + kBucketUnit - 1) / kBucketUnit;
+      // Where many primes lie above the segment, the units that shared memory
+      // bounds (below it) alternate with the wheel tier's, which issue bounds
+      // above it: [9*10^11, 9.1*10^11) 1.459 -> 1.417 ms.  Elsewhere the
+      // heaviest come first ([0, 10^10): 1.075 ms, alternating 1.088).
+      const bool mix = uniform(S.mix) != 0u;
+      const uint32_t nlow = nsmall + nmidu, nwheel = nscan - nlow;
       const uint32_t o = lane & 7u, h = lane >> 3;
       const uint32_t send = sseg + unb;             // shared address past the segment's end
       for (;;) {
@@ -592,6 +599,10 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
         u = uniform(u);
         if (kSolo) u = u * slices + slice;
         if (u >= nunits) break;
+        if (!kSolo && mix && u < nscan) {
+          if (u < 2u * min(nlow, nwheel)) u = (u & 1u) ? nlow + (u >> 1) : u >> 1;
+          else if (nlow > nwheel) u -= nwheel;
+        }
         if (u < nsmall) {
           const bool cst = u < kConstPrimes;
           const uint32_t p = cst ? cTab.p[u] : __ldg(prm.P + u);
