@@ -606,7 +606,9 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
         if (u < nsmall) {
           const bool cst = u < kConstPrimes;
           const uint32_t p = cst ? cTab.p[u] : __ldg(prm.P + u);
-          const uint32_t m = mod_barrett(k0, p, cst ? (uint64_t)cTab.m[u] : __ldg(prm.M + u));
+          const uint64_t M = cst ? (uint64_t)cTab.m[u] : __ldg(prm.M + u);
+          const uint32_t minv = (uint32_t)(M >> 32) + 1u;
+          const uint32_t m = mod_barrett(k0, p, M);
           const uint32_t r = __ldg(prm.R + 8u * u + o);
           uint32_t s = r - m;
           s = min(s, s + p);
@@ -630,7 +632,11 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
           const uint32_t mask = ~(1u << ((c << 3) | o));
           const uint32_t lim = (unb - c + 3u) >> 2;         // word w holds byte 4w + c < nbytes
           const uint32_t w0 = j0 >> 2;
-          const uint32_t n = w0 < lim ? (lim - w0 + p - 1u) / p : 0u;
+          // steps: w0 < p, so floor(whole words / p) or one more (the floor by
+          // a multiplication, exact for factors below 2^16; with a division, a
+          // remainder and two reductions [0, 10^10) took 1.037 ms, now 1.033)
+          const uint32_t nmin = __umulhi(unb >> 2, minv);
+          const uint32_t n = nmin + (w0 + nmin * p < lim ? 1u : 0u);
           const uint32_t pinv = p * (2u - p * p);           // p^-1 mod 64 (p odd, p*p = 1 mod 8)
           const uint32_t u32 = (w0 * pinv) & 31u;
           uint32_t less = 0, same = 0xFFFFFFFFu;             // lanes with a smaller u, with this u
@@ -644,11 +650,10 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
           const uint32_t rank = (uint32_t)__popc(less | (same & ((1u << lane) - 1u)));
           const int off = (int)u32 - (int)rank;
           uint32_t rot = (uint32_t)(__reduce_max_sync(0xFFFFFFFFu, off) - off);
-          if (rot >= n) rot = n ? rot % n : 0u;
+          if (rot >= n) rot = 0;
           const uint32_t first = n - rot;                    // steps before the wrap
           const uint32_t k1 = __reduce_min_sync(0xFFFFFFFFu, first);
-          const uint32_t k2 = __reduce_min_sync(0xFFFFFFFFu, n);
-          const uint32_t k3 = __reduce_max_sync(0xFFFFFFFFu, n);
+          const uint32_t k2 = nmin, k3 = nmin + 1u;
           const uint32_t p4 = 4u * p, turn = n * p4;
           uint32_t q = sseg + 4u * w0 + p4 * rot;
           uint32_t k = 0;
