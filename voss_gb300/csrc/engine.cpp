@@ -324,7 +324,7 @@ void Plan::reserve_capacity(uint32_t max_req, uint64_t max_segs, uint64_t max_bu
     rres.reserve(sizeof(ReqResult) * cap_out);
   }
   cap_bucket = max_bucket_entries;
-  cap_fill = max_bucket_entries ? 65536u : 0u;
+  cap_fill = max_bucket_entries ? 131072u : 0u;
   if (cap_bucket) bucket.reserve(4 * cap_bucket);
   if (cap_fill) fills.reserve(sizeof(FillItem) * cap_fill);
   bcount.reserve(round16(4 * cap_segs));
@@ -517,10 +517,8 @@ void Plan::load_requests(uint32_t n, const uint64_t* a, const uint64_t* b, uint3
       if (bp.cap) {
         // fill items, per window: runs of kFillPrimes primes; a run's hits
         // (8 per p bytes per prime) split over segment ranges so that every
-        // item carries at most about kFillHits hits: items balance, and the
-        // list blocks that the resident fill CTAs are writing at any time
-        // (their items' entries) stay well inside L2, so lines leave it
-        // complete
+        // item carries at most about kFillHits hits, which fit its bins, and
+        // at most kFillSegs segments, which keeps the bins wide
         item_buf.clear();
         std::vector<Window> rw;
         for (uint64_t w0 = 0; w0 < r.nseg; w0 += wsegs) {
@@ -531,7 +529,8 @@ void Plan::load_requests(uint32_t n, const uint64_t* a, const uint64_t* b, uint3
           for (uint32_t p0 = bp.bucket_idx; p0 < r.nprimes; p0 += kFillPrimes) {
             const uint32_t p1 = std::min<uint32_t>(p0 + kFillPrimes, r.nprimes);
             const double hits = per * (E.hInvPrefix[p1] - E.hInvPrefix[p0]);
-            const uint32_t pieces = (uint32_t)std::min<double>(nseg, std::max(1.0, std::ceil(hits / kFillHits)));
+            const uint32_t pieces = (uint32_t)std::min<double>(
+                nseg, std::max<double>((nseg + kFillSegs - 1) / kFillSegs, std::ceil(hits / kFillHits)));
             for (uint32_t j = 0; j < pieces; ++j) {
               const uint32_t g0 = (uint32_t)((uint64_t)nseg * j / pieces);
               const uint32_t g1 = (uint32_t)((uint64_t)nseg * (j + 1) / pieces);
@@ -639,6 +638,7 @@ void Plan::capture(cudaStream_t s) {
   if (graph_exec) return;
   // the kernels' attributes are raised outside the capture
   check_cuda(launch_sieve(prm, 0, threads, s), "sieve attributes");
+  if (cap_fill) check_cuda(launch_bucket_fill(FillParams{}, 0, s), "fill attributes");
   check_cuda(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
   try {
     run_device(s);

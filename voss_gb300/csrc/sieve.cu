@@ -1125,132 +1125,128 @@ finalize_kernel(const ReqDesc* __restrict__ reqs, const BatchHdr* __restrict__ h
 // Bucket fill: one CTA per work item (a request, a run of its bucket primes
 // and a run of its segments; heavy runs of small primes are split over
 // several items so that items carry similar numbers of hits), a thread per
-// prime walking its eight classes.  Pass 1 counts the hits per segment in
-// shared memory; one global atomic per segment reserves room in that
-// segment's list and leaves the reserved base in the shared counter; pass 2
-// walks the hits again and writes each entry at the counter's next slot.  A
-// hit's segment and offset advance by p = pq*S + pr without a division.  A
-// list that would overflow its capacity raises *overflow and drops the entry
-// (the host then reruns without lists).
-//
-// The walk takes the eight classes together, eight independent chains of
-// atomic-then-store per thread: all step unconditionally while all have hits
-// left (each chain's count of hits is known up front), then each finishes
-// under its own predicate.  (Lanes of a warp hold primes of nearly the same size
-// and walk in step, so many of them meet on one segment counter at a time;
-// the counter then hands them consecutive slots and their entries leave in
-// shared sectors.  Spreading the lanes over segments removes the atomic
-// conflicts but scatters the stores, and measured slower.)
-struct FillChain {
-  uint32_t sg, off, n;       // segment (relative to the item's first), offset, hits left
+// prime walking its eight classes as eight independent chains.  A chain is the
+// hit's byte k in the item's segments; its segment is k / S by a
+// multiplication, and its entry goes to the next place of that segment's bin
+// in shared memory.  Then one global atomic per segment reserves room in that
+// segment's list, and a warp per segment copies its bin there.  What bounds
+// it: shared-memory wavefronts and issue, half and half (a returning atomic
+// and a store on random banks per hit).
+// Before, a first walk counted the hits and a second one stored each entry
+// from its lane: 16 write requests per 32 entries (now 3) were the bound, and
+// the chains' segment, offset and count took 23 instructions per hit and walk.
+// [10^14, 10^14 + 10^9): 97 -> 82 us of 342 -> 325; [10^14 - 10^11, 10^14):
+// 26.8 -> 24.4 ms in all.
+// The bins hold 1.54 times an item's expected hits: with at most kFillSegs
+// segments their mean is 54 entries and the margin 4 standard deviations.
+// Primes near sqrt(b) have their hits in clusters (p q = s^2 / 4 - d^2 / 4
+// hardly moves with p for a fixed sum s = p + q), and other items can draw an
+// overfull bin too: such an item walks again and stores its entries from the
+// lanes, at the places that the counts of the first walk reserve.
+// A list that would overflow its capacity raises *overflow and drops the
+// entries past it (the host then reruns without lists).
+struct FillShared {
+  uint32_t cnt[kFillSegs];
+  uint32_t gpos[kFillSegs];      // the next place in the segment's list
+  uint32_t stage[kFillStage];    // the bins, kFillStage / (the item's segments) entries each
 };
-
-template <bool kWrite>
-__device__ __forceinline__ void fill_step(FillChain& c, uint32_t o, uint32_t* cnt, uint32_t* list,
-                                          uint32_t cap, unsigned int* overflow, uint32_t S,
-                                          uint32_t pq, uint32_t pr) {
-  if (kWrite) {
-    const uint32_t pos = atomicAdd(&cnt[c.sg], 1u);
-    if (pos < cap) list[c.sg * cap + pos] = bucket_entry(c.off, o);
-    else atomicOr(overflow, 1u);
-  } else {
-    atomicAdd(&cnt[c.sg], 1u);
-  }
-  c.off += pr;
-  const uint32_t carry = c.off >= S ? 1u : 0u;
-  c.off -= carry ? S : 0u;
-  c.sg += pq + carry;
-}
-
-template <bool kWrite>
-__device__ __forceinline__ void fill_pass(const FillChain (&start)[8], uint32_t* cnt, uint32_t* list,
-                                          uint32_t cap, unsigned int* overflow, uint32_t S,
-                                          uint32_t pq, uint32_t pr) {
-  FillChain c[8];
-  uint32_t all = start[0].n, most = start[0].n;
-#pragma unroll
-  for (int o = 0; o < 8; ++o) { c[o] = start[o]; all = min(all, c[o].n); most = max(most, c[o].n); }
-  for (uint32_t t = 0; t < all; ++t) {
-#pragma unroll
-    for (uint32_t o = 0; o < 8; ++o) fill_step<kWrite>(c[o], o, cnt, list, cap, overflow, S, pq, pr);
-  }
-  for (uint32_t t = all; t < most; ++t) {
-#pragma unroll
-    for (uint32_t o = 0; o < 8; ++o)
-      if (t < c[o].n) fill_step<kWrite>(c[o], o, cnt, list, cap, overflow, S, pq, pr);
-  }
-}
 
 __global__ void __launch_bounds__(kFillPrimes)
 bucket_fill_kernel(const FillParams fp) {
-  __shared__ uint32_t cnt[kMaxBucketSegs];
-  const uint32_t tid = threadIdx.x;
+  extern __shared__ __align__(16) uint32_t smem[];
+  FillShared& sh = *reinterpret_cast<FillShared*>(smem);
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t nitems = fp.nitems ? fp.nitems : fp.hdr->nfill;
   for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
     const FillItem item = fp.items[it];
     const ReqDesc R = fp.reqs[item.req];
     // segments g0..g1 of the window that starts at segment seg0 of the
-    // request; byte offsets below are relative to the window's start k0
+    // request; byte numbers below are relative to segment g0, at k0
     const uint32_t g0 = item.segs & 0xFFFFu, g1 = item.segs >> 16;
     const uint32_t nseg = g1 - g0;
-    const uint32_t S = R.seg_bytes;
-    const uint64_t k0 = R.k_lo + (uint64_t)fp.seg0 * S;
-    const uint32_t total = (uint32_t)min(R.k_hi - k0, (uint64_t)kMaxBucketSegs * S);
-    const uint32_t lo = g0 * S;
-    const uint32_t hi = min(total, g1 * S);
-    const uint32_t cap = R.bucket_cap;
+    const uint32_t cap = R.bucket_cap, S = R.seg_bytes;
+    const uint64_t k0 = R.k_lo + (uint64_t)(fp.seg0 + g0) * S;
+    const uint32_t h = (uint32_t)min(R.k_hi - k0, (uint64_t)nseg * S);
+    // k / S = hi32(k mag) >> shift, exact for k < 2^12 S and S <= 2^19: mag S -
+    // 2^(32 + shift) < S, and 2^12 S S < 2^(32 + shift), 2^shift < S <= 2^(shift + 1)
+    static_assert(kFillSegs < 4096 && kMaxSegBytes <= 1u << 19, "k / S by one multiplication");
+    const uint32_t shift = 31u - (uint32_t)__clz(S - 1u);
+    const uint32_t mag = (uint32_t)(((1ull << (32u + shift)) + S - 1u) / S);
     // the item's lists, segment g at g * cap (the host keeps a window's
     // entries below 2^32)
     uint32_t* const list = fp.bucket + R.bucket_base + (uint64_t)g0 * cap;
     unsigned int* const gcount = fp.bcount + R.seg_base + fp.seg0 + g0;
-    const float inv_s = 1.0f / (float)S;
-    // q = x / S, r = x % S for x < 2^30: a float estimate, corrected once
-    auto divmod_s = [&](uint32_t x, uint32_t& r) {
-      uint32_t q = __float2uint_rz((float)x * inv_s);
-      int32_t d = (int32_t)(x - q * S);
-      if (d < 0) { --q; d += (int32_t)S; } else if (d >= (int32_t)S) { ++q; d -= (int32_t)S; }
-      r = (uint32_t)d;
-      return q;
-    };
-    for (uint32_t g = tid; g < nseg; g += blockDim.x) cnt[g] = 0;
-    __syncthreads();
+    const uint32_t bin = kFillStage / nseg;
+    for (uint32_t g = tid; g < nseg; g += kFillPrimes) sh.cnt[g] = 0;
     const uint32_t i = item.p0 + tid;
-    const bool valid = i < item.p1;
-    uint32_t p = 0, m = 0, pq = 0, pr = 0;
+    uint32_t start[8], step = 0, whole = 0;
     bool low = false;
-    if (valid) {
-      p = __ldg(fp.P + i);
-      m = mod_barrett(k0, p, __ldg(fp.M + i));
-      low = 30ull * k0 < (uint64_t)p * p;
-      pq = divmod_s(p, pr);
-    }
-    // first hit at or after byte lo of each class and the number of hits
-    // below hi, kept for both passes; the eight residue loads issue together
-    uint32_t r8[8];
-    if (valid) load_residues(fp.R, i, r8);
-    FillChain ch[8];
 #pragma unroll
-    for (int o = 0; o < 8; ++o) {
-      ch[o].sg = 0; ch[o].off = 0; ch[o].n = 0;
-      if (valid) {
-        const uint32_t r = r8[o];
-        uint32_t k = r >= m ? r - m : r + p - m;
-        if (low) k = lift_to_square(k, k0, p, o, total);
-        if (k < lo) k += ((lo - k + p - 1) / p) * p;
-        if (k < hi) {
-          ch[o].n = (hi - 1u - k) / p + 1u;
-          ch[o].sg = divmod_s(k, ch[o].off) - g0;
+    for (int o = 0; o < 8; ++o) start[o] = h;
+    if (i < item.p1) {
+      load_residues(fp.R, i, start);
+      const uint32_t p = __ldg(fp.P + i);
+      const uint32_t m = mod_barrett(k0, p, __ldg(fp.M + i));
+      low = 30ull * k0 < (uint64_t)p * p;
+      step = min(p, h);                            // (k stays below 2 h)
+      whole = low ? 0u : h / p;
+#pragma unroll
+      for (int o = 0; o < 8; ++o) {
+        start[o] = start[o] >= m ? start[o] - m : start[o] + p - m;
+        if (low) start[o] = lift_to_square(start[o], k0, p, o, h);
+        start[o] = min(start[o], h);
+      }
+    }
+    __syncthreads();
+    {
+      uint32_t k[8];
+#pragma unroll
+      for (int o = 0; o < 8; ++o) k[o] = start[o];
+      auto put = [&](uint32_t x, uint32_t o) {
+        const uint32_t g = __umulhi(x, mag) >> shift;
+        const uint32_t pos = min(atomicAdd(&sh.cnt[g], 1u), bin - 1u);
+        sh.stage[g * bin + pos] = bucket_entry(x - g * S, o);
+      };
+      for (uint32_t t = 0; t < whole; ++t) {
+#pragma unroll
+        for (uint32_t o = 0; o < 8; ++o) { put(k[o], o); k[o] += step; }
+      }
+      do {
+#pragma unroll
+        for (uint32_t o = 0; o < 8; ++o)
+          if (k[o] < h) { put(k[o], o); k[o] += step; }
+      } while (low && min(min(min(k[0], k[1]), min(k[2], k[3])), min(min(k[4], k[5]), min(k[6], k[7]))) < h);
+    }
+    __syncthreads();
+    bool mine = false;
+    for (uint32_t g = tid; g < nseg; g += kFillPrimes) mine |= sh.cnt[g] > bin;
+    const bool full = __syncthreads_or(mine);
+    for (uint32_t g = tid; g < nseg; g += kFillPrimes) {
+      const uint32_t c = sh.cnt[g];
+      const uint32_t at = c ? atomicAdd(gcount + g, c) : 0u;
+      if (at + c > cap) atomicOr(fp.overflow, 1u);
+      sh.gpos[g] = at;
+    }
+    __syncthreads();
+    if (!full) {
+      for (uint32_t g = warp; g < nseg; g += kFillPrimes / 32) {
+        const uint32_t at = sh.gpos[g], n = min(sh.cnt[g], cap - min(at, cap));
+        uint32_t* const to = list + ((uint64_t)g * cap + at);
+        const uint32_t* const from = sh.stage + g * bin;
+#pragma unroll 2
+        for (uint32_t e = lane; e < n; e += 32) to[e] = from[e];
+      }
+    } else {
+#pragma unroll
+      for (uint32_t o = 0; o < 8; ++o) {
+#pragma unroll 1
+        for (uint32_t k = start[o]; k < h; k += step) {
+          const uint32_t g = __umulhi(k, mag) >> shift;
+          const uint32_t pos = atomicAdd(&sh.gpos[g], 1u);
+          if (pos < cap) list[(uint64_t)g * cap + pos] = bucket_entry(k - g * S, o);
         }
       }
     }
-    fill_pass<false>(ch, cnt, list, cap, fp.overflow, S, pq, pr);
-    __syncthreads();
-    for (uint32_t g = tid; g < nseg; g += blockDim.x) {
-      const uint32_t c = cnt[g];
-      cnt[g] = c ? atomicAdd(gcount + g, c) : 0u;
-    }
-    __syncthreads();
-    fill_pass<true>(ch, cnt, list, cap, fp.overflow, S, pq, pr);
     __syncthreads();
   }
 }
@@ -1411,16 +1407,31 @@ cudaError_t launch_zero(ZeroSpan z0, ZeroSpan z1, ZeroSpan z2, uint32_t max_grid
   return cudaGetLastError();
 }
 
+// the attribute is per device, as in launch_sieve
+static cudaError_t fill_attributes() {
+  static AttrCache attr;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  return (cudaError_t)attr.ensure(dev, sizeof(FillShared), [](size_t n) {
+    return (int)cudaFuncSetAttribute(bucket_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+  });
+}
+
 uint32_t bucket_fill_ctas_per_sm() {
   static int n = 0;
-  if (!n && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bucket_fill_kernel, kFillPrimes, 0) != cudaSuccess || n < 1))
+  if (!n && (fill_attributes() != cudaSuccess ||
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bucket_fill_kernel, kFillPrimes, sizeof(FillShared)) !=
+                 cudaSuccess ||
+             n < 1))
     n = 1;
   return (uint32_t)n;
 }
 
 cudaError_t launch_bucket_fill(const FillParams& fp, uint32_t grid, cudaStream_t stream) {
+  if (cudaError_t e = fill_attributes()) return e;
   if (grid == 0) return cudaSuccess;
-  bucket_fill_kernel<<<grid, kFillPrimes, 0, stream>>>(fp);
+  bucket_fill_kernel<<<grid, kFillPrimes, sizeof(FillShared), stream>>>(fp);
   return cudaGetLastError();
 }
 

@@ -238,7 +238,12 @@ constexpr uint32_t kMaxBucketSegs = 4096;
 constexpr uint32_t kWheelUnitLog2Max = 10;
 constexpr uint32_t kBucketUnit = 1024;       // list entries per work unit of the sieve kernel
 constexpr uint32_t kFillPrimes = 256;        // bucket primes per fill work item
-constexpr uint32_t kFillHits = 16384;        // list entries per fill work item, about
+// An item's hits (about), its bins and its segments: 55 KB of shared memory, so
+// that four fill CTAs share an SM.  [10^14 - 10^11, 10^14): 24.4 ms, with 6144
+// hits 24.6, 15360 (two CTAs) 25.4, 5120 26.4.
+constexpr uint32_t kFillHits = 8704;
+constexpr uint32_t kFillStage = 13440;
+constexpr uint32_t kFillSegs = 160;
 
 // A bucket list entry: the segment-local bit index 8 * byte + class, so that
 // entry / 32 is the word and entry mod 32 the bit within it.
