@@ -818,6 +818,8 @@ constexpr uint32_t kSoloSlicePrimes = 256;
 // the fill is far cheaper.
 constexpr uint32_t kSoloListPrimes = 100000;
 constexpr uint32_t kSoloLargeCap = 1u << 14;
+// Segments of a lone_kernel run: 8 MB of records, ranges up to 1.7 * 10^12 wide.
+constexpr uint64_t kLoneMaxSegs = 1u << 18;
 
 bool Engine::solo_start(uint64_t a, uint64_t b, bool gaps, uint32_t* bitmap) {
   if (b <= a || b > kMaxB) return false;
@@ -825,18 +827,18 @@ bool Engine::solo_start(uint64_t a, uint64_t b, bool gaps, uint32_t* bitmap) {
   const Config c = tuned_for(a, b, false);
   const ReqDesc r = describe(a, b, gaps ? kReqGaps : 0u, c);
   const uint64_t ctas = std::min<uint64_t>((uint64_t)sm_count * cfg.ctas_per_sm, kSoloMaxSegs);
-  if (r.nseg > ctas) return false;
+  const bool waves = r.nseg > ctas;          // more segments than CTAs: lone_kernel
+  if (waves && (bitmap || r.nseg > kLoneMaxSegs)) return false;
   uint64_t slices = 1;
   if (r.nseg * r.seg_bytes <= kSoloMergeBytes)
     slices = std::max<uint64_t>(1, std::min<uint64_t>(ctas / r.nseg, r.nprimes / kSoloSlicePrimes));
   // (runs with a bitmap never take lists)
   const BucketPlan bp = bucket_plan(c, b, r.nprimes, r.nseg, r.seg_bytes);
-  if (bp.cap && !bitmap && (!cfg.auto_tune || (r.nprimes - bp.bucket_idx) / slices > kSoloListPrimes)) return false;
+  if (bp.cap && !bitmap && (waves || !cfg.auto_tune || (r.nprimes - bp.bucket_idx) / slices > kSoloListPrimes)) return false;
 
   if (!solo.clean) {
     solo.ctl.reserve(sizeof(SoloCtl));
     solo.acc.reserve(sizeof(ReqAccum));
-    solo.segs.reserve(sizeof(SegRec) * kSoloMaxSegs);
     solo.merge.reserve(kSoloMergeBytes);
     solo.large.reserve(sizeof(LargeGapRec) * kSoloLargeCap);
     solo.out.reserve(sizeof(SoloResult));
@@ -844,6 +846,7 @@ bool Engine::solo_start(uint64_t a, uint64_t b, bool gaps, uint32_t* bitmap) {
     check_cuda(cudaMemsetAsync(solo.acc.ptr, 0, sizeof(ReqAccum), stream), "solo accumulators");
     check_cuda(cudaMemsetAsync(solo.merge.ptr, 0xFF, kSoloMergeBytes, stream), "solo words");
   }
+  solo.segs.reserve(sizeof(SegRec) * std::max<uint64_t>(r.nseg, kSoloMaxSegs));
   SieveParams prm = table_params();
   prm.seg_bytes = r.seg_bytes;
   prm.segs = solo.segs.as<SegRec>();
@@ -863,7 +866,10 @@ bool Engine::solo_start(uint64_t a, uint64_t b, bool gaps, uint32_t* bitmap) {
   prm.flags = bitmap ? kFlagBitmap : 0u;
   prm.bitmap = bitmap;
   solo.clean = false;                        // until the run has ended well
-  check_cuda(launch_solo(prm, cfg.threads, stream), "solo_kernel");
+  if (waves)
+    check_cuda(launch_lone(prm, (uint32_t)ctas, cfg.threads, stream), "lone_kernel");
+  else
+    check_cuda(launch_solo(prm, cfg.threads, stream), "solo_kernel");
   return true;
 }
 
@@ -877,8 +883,7 @@ const ReqResult* Engine::run_solo(uint64_t a, uint64_t b, std::vector<LargeGapRe
   check_cuda(cudaStreamSynchronize(stream), "sieve run");
   const SoloResult* out = solo_done();
   if (lg) {
-    if (out->n_large > kSoloLargeCap)
-      throw Error(VOSS_ERR_INTERNAL, "large-gap buffer overflow (" + std::to_string(out->n_large) + " gaps)");
+    if (out->n_large > kSoloLargeCap) return nullptr;      // (a plan's buffer is larger)
     lg->resize(out->n_large);
     if (out->n_large)
       check_cuda(cudaMemcpy(lg->data(), solo.large.ptr, sizeof(LargeGapRec) * out->n_large, cudaMemcpyDeviceToHost),

@@ -312,6 +312,7 @@ size_t sieve_static_smem_bytes();      // the sieve kernel's static shared memor
 cudaError_t launch_sieve(const SieveParams& prm, uint32_t grid, uint32_t threads,
                          cudaStream_t stream);
 cudaError_t launch_solo(const SieveParams& prm, uint32_t threads, cudaStream_t stream);
+cudaError_t launch_lone(const SieveParams& prm, uint32_t grid, uint32_t threads, cudaStream_t stream);
 cudaError_t launch_bucket_fill(const FillParams& fp, uint32_t grid, cudaStream_t stream);
 uint32_t bucket_fill_ctas_per_sm();      // resident fill CTAs per SM (occupancy query, cached)
 // Cut a batch's ranges at every endpoint into the disjoint pieces some range

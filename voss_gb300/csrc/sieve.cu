@@ -279,6 +279,31 @@ __device__ __noinline__ void claim_item(unsigned long long* queue, const ReqDesc
   }
 }
 
+// The same for a lone request without lists (lone_kernel): the next of its
+// segments and the table primes with p*p below the segment's upper end.
+__device__ __noinline__ void claim_lone(const SieveParams& prm, SegItem& d, uint32_t lane) {
+  const ReqDesc& R = prm.solo;
+  unsigned long long it = 0;
+  if (lane == 0) it = atomicAdd(&prm.ctl->queue, 1ull);
+  const uint64_t si = __shfl_sync(0xFFFFFFFFu, it, 0);
+  if (si >= R.nseg) {
+    if (lane == 0) d.valid = 0;
+    return;
+  }
+  const uint64_t k0 = R.k_lo + si * R.seg_bytes;
+  const uint32_t nb = (uint32_t)min((uint64_t)R.seg_bytes, R.k_hi - k0);
+  const uint64_t hi_num = 30ull * (k0 + nb);
+  const uint32_t np = warp_count_leading(R.nprimes, lane, [&](uint32_t i) {
+    const uint64_t p = prm.P[i];
+    return p * p < hi_num;
+  });
+  if (lane == 0) {
+    d.k0 = k0; d.nbytes = nb; d.item = si; d.valid = 1; d.req = 0; d.np = np; d.bcnt = 0; d.bbase = 0;
+    d.mix = np && prm.P[np - 1u] >= 2u * nb;
+    set_item(d, R, si == 0 ? prm.keep0 : ~0u, si + 1u == R.nseg ? prm.keepl : ~0u);
+  }
+}
+
 // Shared-memory per-warp record used to stitch warps inside a segment.
 struct WarpRec {
   uint32_t first1, last1;    // relative value + 1 (0 = none)
@@ -395,9 +420,14 @@ __device__ __forceinline__ void finalize_request(const ReqDesc& R, uint32_t r, c
   }
 }
 
-// kSolo: the one-launch form for a lone request, see solo_kernel.
-template <bool kSolo>
+// The three forms of the sieve: work items of a plan's requests, and a lone
+// request in one launch, with at most a wave of segments (solo_kernel) or with
+// more (lone_kernel).
+constexpr int kFormBatch = 0, kFormSolo = 1, kFormLone = 2;
+
+template <int kForm>
 __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
+  constexpr bool kSolo = kForm == kFormSolo;
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* seg = smem;
   const uint32_t sseg = (uint32_t)__cvta_generic_to_shared(seg);
@@ -475,6 +505,8 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       set_item(d, R, si == 0 ? prm.keep0 : ~0u, si + 1u == (uint32_t)R.nseg ? prm.keepl : ~0u);
       s_item[1].valid = 0;
     }
+  } else if constexpr (kForm == kFormLone) {
+    if (warp == 0) claim_lone(prm, s_item[0], lane);
   } else {
     const uint64_t total_segs = prm.hdr->total_segs;
     item_end = prm.item_hi ? min(total_segs, prm.item_hi) : total_segs;
@@ -581,9 +613,13 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       const uint32_t k0s = uniform((uint32_t)(k0 >> 10)), k0l = uniform((uint32_t)k0);
       const uint32_t bcnt = uniform(S.bcnt);
       const uint64_t bbase = S.bbase;
-      if (!kSolo && warp == 0)                      // overlaps the marking
-        claim_item(prm.queue, prm.reqs, prm.P, prm.bcount, prm.item_lo, item_end, prm.list_seg0, nreq,
-                   s_item[cur ^ 1u], lane);
+      if (!kSolo && warp == 0) {                    // overlaps the marking
+        if constexpr (kForm == kFormLone)
+          claim_lone(prm, s_item[cur ^ 1u], lane);
+        else
+          claim_item(prm.queue, prm.reqs, prm.P, prm.bcount, prm.item_lo, item_end, prm.list_seg0, nreq,
+                     s_item[cur ^ 1u], lane);
+      }
       const uint32_t nunits = nscan + (bcnt + kBucketUnit - 1) / kBucketUnit;
       // Where many primes lie above the segment, the units that shared memory
       // bounds (below it) alternate with the wheel tier's, which issue bounds
@@ -897,7 +933,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       if (wbeg < wend && wend == nwords) seg[nwords - 1u] &= S.keepl;
       if (prm.flags & kFlagBitmap) {
         __syncthreads();
-        uint32_t* dst = prm.bitmap + ((k0 - (kSolo ? prm.solo.k_lo : prm.reqs[0].k_lo)) >> 2);
+        uint32_t* dst = prm.bitmap + ((k0 - (kForm != kFormBatch ? prm.solo.k_lo : prm.reqs[0].k_lo)) >> 2);
         for (uint32_t w = tid; w < nwords; w += nthr) dst[w] = seg[w];
       }
       GapSink sk;
@@ -1071,15 +1107,17 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
   }
   __syncthreads();
   if (cur_req >= 0 && cur_gaps) flush();
-  if constexpr (kSolo) {
-    // the last segment to be reduced writes the result and leaves the
-    // accumulators and the control words clear for the next run
-    if (prm.solo.nseg > 1) {
+  if constexpr (kForm != kFormBatch) {
+    // the last segment to be reduced (the last CTA to run out of segments)
+    // writes the result and leaves the accumulators and the control words
+    // clear for the next run
+    const uint32_t parts = kSolo ? (uint32_t)prm.solo.nseg : gridDim.x;
+    if (parts > 1) {
       __threadfence();
       __syncthreads();
       if (tid == 0) s_ctr = atomicAdd(&prm.ctl->done, 1u);
       __syncthreads();
-      if (s_ctr != (uint32_t)prm.solo.nseg - 1u) return;
+      if (s_ctr != parts - 1u) return;
       __threadfence();
     } else {
       __syncthreads();
@@ -1092,12 +1130,13 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       prm.out->n_large = __ldcg(&prm.ctl->n_large);
       prm.ctl->n_large = 0;
       prm.ctl->done = 0;
+      prm.ctl->queue = 0;
     }
   }
 }
 
 __global__ void __launch_bounds__(kMaxThreads, 1) sieve_segments_kernel(const SieveParams prm) {
-  sieve_body<false>(prm);
+  sieve_body<kFormBatch>(prm);
 }
 
 // A lone request in one launch.  A range of one wave or less leaves most of
@@ -1108,7 +1147,18 @@ __global__ void __launch_bounds__(kMaxThreads, 1) sieve_segments_kernel(const Si
 // segment, and the last segment writes the result to host memory.  No CTA
 // waits for another.
 __global__ void __launch_bounds__(kMaxThreads, 1) solo_kernel(const __grid_constant__ SieveParams prm) {
-  sieve_body<true>(prm);
+  sieve_body<kFormSolo>(prm);
+}
+
+// A lone request of more segments than a wave, without lists, in one launch:
+// one CTA per SM takes segments from a queue, and the last CTA to find it empty
+// writes the result to host memory.  As a plan the same request took a copy up,
+// a zeroing launch, the sieve, a launch of one block that folds the records
+// and two copies down with a wait each: Context(10^10) 1079 -> 1052 us, 2*10^9
+// numbers at 0 234 -> 221, Context(10^12) 125.5 -> 124.3 ms (one block folded
+// its 150 000 records).
+__global__ void __launch_bounds__(kMaxThreads, 1) lone_kernel(const __grid_constant__ SieveParams prm) {
+  sieve_body<kFormLone>(prm);
 }
 
 __global__ void __launch_bounds__(256)
@@ -1389,6 +1439,20 @@ cudaError_t launch_solo(const SieveParams& prm, uint32_t threads, cudaStream_t s
   });
   if (rc) return (cudaError_t)rc;
   solo_kernel<<<(uint32_t)prm.solo.nseg * prm.slices, threads, smem, stream>>>(prm);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_lone(const SieveParams& prm, uint32_t grid, uint32_t threads, cudaStream_t stream) {
+  const size_t smem = std::max(sieve_smem_bytes(prm.seg_bytes, threads), sizeof(uint32_t) * (size_t)kFinalWords);
+  static AttrCache attr;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const int rc = attr.ensure(dev, smem, [](size_t n) {
+    return (int)cudaFuncSetAttribute(lone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+  });
+  if (rc) return (cudaError_t)rc;
+  lone_kernel<<<grid, threads, smem, stream>>>(prm);
   return cudaGetLastError();
 }
 

@@ -327,9 +327,9 @@ struct SoloResult {
 constexpr uint32_t kSoloMaxSegs = 1024;
 struct SoloCtl {
   uint32_t seg_done[kSoloMaxSegs];   // slices of each segment that are merged
-  uint32_t done;                     // segments that are reduced
+  uint32_t done;                     // segments that are reduced; CTAs without a segment left
   uint32_t n_large;
-  uint32_t pad[2];
+  unsigned long long queue;          // lone_kernel: the next segment
 };
 
 struct SieveParams {
@@ -359,8 +359,8 @@ struct SieveParams {
   // a request sits at slot si - list_seg0 (the window's first segment).
   uint64_t item_lo, item_hi;
   uint64_t list_seg0;
-  // The one-launch form (solo_kernel): a lone request without lists whose
-  // segments fit one CTA per SM each, slices CTAs sharing a segment's primes.
+  // The one-launch forms: a lone request without lists.  solo_kernel: its
+  // segments fit one CTA per SM each, slices CTAs share a segment's primes.
   ReqDesc solo;
   uint32_t slices;
   uint32_t low_k;            // wheel byte past every prime that may sieve (rounded to a row)
