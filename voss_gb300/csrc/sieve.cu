@@ -422,12 +422,12 @@ __device__ __forceinline__ void finalize_request(const ReqDesc& R, uint32_t r, c
 
 // The three forms of the sieve: work items of a plan's requests, and a lone
 // request in one launch, with at most a wave of segments (solo_kernel) or with
-// more (lone_kernel).
-constexpr int kFormBatch = 0, kFormSolo = 1, kFormLone = 2;
+// more (lone_kernel), there with gaps or counts alone.
+constexpr int kFormBatch = 0, kFormSolo = 1, kFormLone = 2, kFormLoneCount = 3;
 
 template <int kForm>
 __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
-  constexpr bool kSolo = kForm == kFormSolo;
+  constexpr bool kSolo = kForm == kFormSolo, kLone = kForm == kFormLone || kForm == kFormLoneCount;
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* seg = smem;
   const uint32_t sseg = (uint32_t)__cvta_generic_to_shared(seg);
@@ -441,6 +441,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
   // waits on that lookup)
   __shared__ SegItem s_item[2];
   __shared__ uint32_t s_ctr;
+  __shared__ uint32_t s_filled;                    // the segment in hand has been filled by the warps
 
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t nthr = blockDim.x, nwarps = nthr >> 5;
@@ -449,7 +450,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
   for (uint32_t i = tid; i < kSmemHistCopies * kByteValues; i += nthr) bhist[i] = 0;
   for (uint32_t x = tid; x < kByteValues; x += nthr)
     btab[x] = x ? (uint8_t)((__ffs(x) - 1) | ((31 - __clz(x)) << 4)) : 0;
-  if (tid == 0) s_ctr = 0;
+  if (tid == 0) s_ctr = s_filled = 0;
   int cur_req = -1;
   bool cur_gaps = false;
   // Add the histograms to the current request's accumulators and clear them:
@@ -489,6 +490,34 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
     }
   };
 
+  // The presieve tiles' AND in 16-byte units v, v + step, .. below end of the
+  // segment at k0 (up to 3 words past its end: never read), and in the solo
+  // form into the words that the slices left.
+  auto fill = [&](uint64_t k0, uint32_t v, uint32_t end, uint32_t step, const uint32_t* merged) {
+    // copy (phase mod 16) of each tile holds the phase on a 16-byte boundary
+    uint32_t toff[kTiles];                         // 16-byte units from each tile's start
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t) {
+      const uint32_t ph = (uint32_t)(k0 % tile_period(t));
+      toff[t] = (ph & 15u) * prm.tile_stride16[t] + (ph >> 4);
+    }
+    uint4* seg4 = reinterpret_cast<uint4*>(seg);
+#pragma unroll 4
+    for (; v < end; v += step) {
+      uint4 x = __ldg(reinterpret_cast<const uint4*>(prm.tile[0]) + toff[0] + v);
+#pragma unroll
+      for (int t = 1; t < kTiles; ++t) {
+        const uint4 y = __ldg(reinterpret_cast<const uint4*>(prm.tile[t]) + toff[t] + v);
+        x.x &= y.x; x.y &= y.y; x.z &= y.z; x.w &= y.w;
+      }
+      if (kSolo && merged) {
+        const uint4 y = __ldcg(reinterpret_cast<const uint4*>(merged) + v);
+        x.x &= y.x; x.y &= y.y; x.z &= y.z; x.w &= y.w;
+      }
+      seg4[v] = x;
+    }
+  };
+
   uint64_t item_end = 0;
   uint32_t nreq = 1, cur = 0;
   // solo: this CTA's segment and its share of the segment's units
@@ -505,7 +534,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       set_item(d, R, si == 0 ? prm.keep0 : ~0u, si + 1u == (uint32_t)R.nseg ? prm.keepl : ~0u);
       s_item[1].valid = 0;
     }
-  } else if constexpr (kForm == kFormLone) {
+  } else if constexpr (kLone) {
     if (warp == 0) claim_lone(prm, s_item[0], lane);
   } else {
     const uint64_t total_segs = prm.hdr->total_segs;
@@ -515,9 +544,9 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       claim_item(prm.queue, prm.reqs, prm.P, prm.bcount, prm.item_lo, item_end, prm.list_seg0, nreq, s_item[0], lane);
   }
   __syncthreads();
-  // Three barriers per segment: after the fill, after the marking, before
-  // the warps are stitched.  No thread reads the segment after the last one,
-  // so the next fill follows it directly.
+  // Two or three barriers per segment: after a fill by all threads, after the
+  // marking, before the warps are stitched.  No thread reads the segment after
+  // the last one, so the next fill or marking follows it directly.
   for (;; cur ^= 1u) {
     // work queue: the next (request, segment) item, heaviest requests first
     const SegItem& S = s_item[cur];
@@ -535,43 +564,20 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
         flush();
       }
       cur_req = (int)req;
-      cur_gaps = (S.rflags & kReqGaps) != 0;
+      cur_gaps = kLone ? kForm == kFormLone : (S.rflags & kReqGaps) != 0;
     }
 
-    // 1. presieve fill, of all words or (solo, after the slices are merged)
+    // 1. presieve fill, of all words (unless the warps have filled them after
+    //    scanning the segment before) or, solo, after the slices are merged,
     //    into what the slices left
-    auto fill = [&](const uint32_t* merged) {
-      // copy (phase mod 16) of each tile holds the phase on a 16-byte boundary
-      uint32_t toff[kTiles];                       // 16-byte units from each tile's start
-#pragma unroll
-      for (int t = 0; t < kTiles; ++t) {
-        const uint32_t ph = (uint32_t)(k0 % tile_period(t));
-        toff[t] = (ph & 15u) * prm.tile_stride16[t] + (ph >> 4);
-      }
-      uint4* seg4 = reinterpret_cast<uint4*>(seg);
-      const uint32_t n16 = (nbytes + 15u) >> 4;    // up to 3 words past the end: never read
-#pragma unroll 4
-      for (uint32_t v = tid; v < n16; v += nthr) {
-        uint4 x = __ldg(reinterpret_cast<const uint4*>(prm.tile[0]) + toff[0] + v);
-#pragma unroll
-        for (int t = 1; t < kTiles; ++t) {
-          const uint4 y = __ldg(reinterpret_cast<const uint4*>(prm.tile[t]) + toff[t] + v);
-          x.x &= y.x; x.y &= y.y; x.z &= y.z; x.w &= y.w;
-        }
-        if (kSolo && merged) {
-          const uint4 y = __ldcg(reinterpret_cast<const uint4*>(merged) + v);
-          x.x &= y.x; x.y &= y.y; x.z &= y.z; x.w &= y.w;
-        }
-        seg4[v] = x;
-      }
-    };
     if (kSolo && slices > 1u) {
       const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
       for (uint32_t v = tid; v < (nbytes + 15u) >> 4; v += nthr) reinterpret_cast<uint4*>(seg)[v] = ones;
-    } else {
-      fill(nullptr);
+      __syncthreads();
+    } else if (kSolo || !s_filled) {
+      fill(k0, tid, (nbytes + 15u) >> 4, nthr, nullptr);
+      __syncthreads();
     }
-    __syncthreads();
 
     // 2. marking.  Work units handed out by a shared counter:
     //    units [0, nsmall): one prime each, p < split: a warp per prime, lane
@@ -614,7 +620,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       const uint32_t bcnt = uniform(S.bcnt);
       const uint64_t bbase = S.bbase;
       if (!kSolo && warp == 0) {                    // overlaps the marking
-        if constexpr (kForm == kFormLone)
+        if constexpr (kLone)
           claim_lone(prm, s_item[cur ^ 1u], lane);
         else
           claim_item(prm.queue, prm.reqs, prm.P, prm.bcount, prm.item_lo, item_end, prm.list_seg0, nreq,
@@ -903,7 +909,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       __syncthreads();
       if (s_ctr != slices - 1u) return;
       __threadfence();
-      fill(words);
+      fill(k0, tid, (nbytes + 15u) >> 4, nthr, words);
       __syncthreads();
       uint4* const w4 = reinterpret_cast<uint4*>(words);
       for (uint32_t v = tid; v < (nbytes + 15u) >> 4; v += nthr) w4[v] = make_uint4(~0u, ~0u, ~0u, ~0u);
@@ -943,7 +949,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       sk.req = req; sk.base = 30ull * k0;
       const uint32_t m41 = (k0 & 1ull) ? 0x99669966u : 0x66996699u;
       uint32_t first1 = 0, last1 = 0, cnt = 0, c41 = 0, c31 = 0, maxg = 0, maxgs = 0;
-      const bool gaps = uniform(S.rflags & kReqGaps) != 0;
+      const bool gaps = kLone ? kForm == kFormLone : uniform(S.rflags & kReqGaps) != 0;
       if (gaps) {
         // Byte by byte, four fixed steps per word, so the lanes of a warp
         // stay in step whatever their primes.  A byte's value is counted in
@@ -1063,6 +1069,22 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
         r.maxg = gm; r.maxgs = gs; r.pad = 0;
         wrec[warp] = r;
       }
+      // After a gap scan a warp fills its words for the next segment, where
+      // that has runs as long (and no other warp still copies them out): the
+      // fill's loads from L2 overlap the other warps' scan, and the segment
+      // needs a barrier less (10^10 numbers at 0 1.033 -> 1.023 ms, at 10^12
+      // 1.383 -> 1.372).  After a count's short scan, which leaves little to
+      // overlap, filling in turn costs 0.5 % more than all threads do.
+      if constexpr (!kSolo && kForm != kFormLoneCount) {
+        const SegItem& N = s_item[cur ^ 1u];
+        const bool filled = gaps && N.valid && !(prm.flags & kFlagBitmap) &&
+                            ((((N.nbytes + 3u) >> 2) + nthr - 1) / nthr | 1u) == run;
+        if (tid == 0) s_filled = filled;
+        if (filled) {
+          __syncwarp();
+          fill(N.k0, 8u * run * warp + lane, min(8u * run * (warp + 1u), (N.nbytes + 15u) >> 4), 32u, nullptr);
+        }
+      }
       __syncthreads();
       // warps are stitched like lanes, lane = warp: the gap from the last
       // prime before a warp to its first prime, the largest gap (ties: the
@@ -1159,6 +1181,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) solo_kernel(const __grid_const
 // its 150 000 records).
 __global__ void __launch_bounds__(kMaxThreads, 1) lone_kernel(const __grid_constant__ SieveParams prm) {
   sieve_body<kFormLone>(prm);
+}
+// The same for counts alone: without the gap scan's code in the kernel a count
+// of [0, 3*10^10) takes 2456 us instead of 2462.
+__global__ void __launch_bounds__(kMaxThreads, 1) lone_count_kernel(const __grid_constant__ SieveParams prm) {
+  sieve_body<kFormLoneCount>(prm);
 }
 
 __global__ void __launch_bounds__(256)
@@ -1444,15 +1471,19 @@ cudaError_t launch_solo(const SieveParams& prm, uint32_t threads, cudaStream_t s
 
 cudaError_t launch_lone(const SieveParams& prm, uint32_t grid, uint32_t threads, cudaStream_t stream) {
   const size_t smem = std::max(sieve_smem_bytes(prm.seg_bytes, threads), sizeof(uint32_t) * (size_t)kFinalWords);
-  static AttrCache attr;
+  const bool gaps = (prm.solo.rflags & kReqGaps) != 0;
+  static AttrCache attr, attr_count;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const int rc = attr.ensure(dev, smem, [](size_t n) {
+  const int rc = gaps ? attr.ensure(dev, smem, [](size_t n) {
     return (int)cudaFuncSetAttribute(lone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+  }) : attr_count.ensure(dev, smem, [](size_t n) {
+    return (int)cudaFuncSetAttribute(lone_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
   });
   if (rc) return (cudaError_t)rc;
-  lone_kernel<<<grid, threads, smem, stream>>>(prm);
+  if (gaps) lone_kernel<<<grid, threads, smem, stream>>>(prm);
+  else lone_count_kernel<<<grid, threads, smem, stream>>>(prm);
   return cudaGetLastError();
 }
 
