@@ -6,7 +6,9 @@
 //   * the sieving-prime table (primes >= 61, with Barrett constants and the
 //     eight residue-class starts of each prime) is built once per process and
 //     stays resident on the device, growing on demand up to sqrt(10^14+10^10);
-//   * a run is two kernel launches for any number of ranges and segments,
+//   * a lone range without bucket lists is one kernel launch that writes its
+//     result to host memory; a run of any number of ranges is three (zeroing,
+//     sieve, finalize) and the bucket fill where lists are used; either way
 //     with no per-segment host work, no per-prime launches and no
 //     synchronisation until the results are read;
 //   * all buffers are reused across calls (grow-only).

@@ -20,13 +20,15 @@
 //      set again;
 //   3. reduce in the same CTA: popcount (count), masked popcount (p mod 4,
 //      p mod 3), and an ordered gap scan with a warp max-scan carrying the
-//      previous prime, histogram in shared memory -- replaces extract +
+//      previous prime, byte values and gaps counted in shared memory -- replaces extract +
 //      thrust::sort + mod4 + gaps kernels (extract.cu:10-39,
 //      chebyshev.cu:11-25, gaps.cu:31-75).  Count-only requests skip the
 //      gap scan.
 // Segment boundaries, 2/3/5 and request totals are stitched by
 // finalize_kernel (the reference does this on the host, context.cu:462-524);
-// combine_kernel rebuilds requests that shared atoms of a batch.
+// combine_kernel rebuilds requests that shared atoms of a batch.  A lone request
+// without lists runs in one launch: solo_kernel with at most a wave of segments,
+// lone_kernel or lone_count_kernel with more.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1188,7 +1190,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1) lone_count_kernel(const __grid
   sieve_body<kFormLoneCount>(prm);
 }
 
-__global__ void __launch_bounds__(256)
+// A CTA per request; a lone one's records are folded by 1024 threads instead of
+// 256 (150 000 records: 0.54 -> 0.18 ms).
+__global__ void __launch_bounds__(kMaxThreads)
 finalize_kernel(const ReqDesc* __restrict__ reqs, const BatchHdr* __restrict__ hdr,
                 const SegRec* __restrict__ segs, ReqAccum* __restrict__ acc, LargeGapRec* large,
                 unsigned int* n_large, uint32_t large_cap, ReqResult* __restrict__ out) {
@@ -1535,7 +1539,7 @@ cudaError_t launch_finalize(const ReqDesc* reqs, const BatchHdr* hdr, const SegR
                             uint32_t large_cap, ReqResult* out, uint32_t grid,
                             cudaStream_t stream) {
   if (grid == 0) return cudaSuccess;
-  finalize_kernel<<<grid, 256, 0, stream>>>(reqs, hdr, segs, acc, large, n_large, large_cap, out);
+  finalize_kernel<<<grid, grid == 1 ? 1024 : 256, 0, stream>>>(reqs, hdr, segs, acc, large, n_large, large_cap, out);
   return cudaGetLastError();
 }
 
