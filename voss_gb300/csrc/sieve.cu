@@ -106,15 +106,12 @@ __device__ __forceinline__ void and_word_if(uint32_t a, uint32_t mask, bool on) 
                :: "r"(a), "r"(mask), "r"((uint32_t)on) : "memory");
 }
 
-// The same for a candidate given as bit index v = 8 * byte + class of the
-// segment at shared address seg: its word is v / 32 and its mask 0xFFFFFFFE
-// rotated by v (a funnel shift takes its count mod 32).
-__device__ __forceinline__ void clear_bit(uint32_t seg, uint32_t v) {
-  and_word(seg + 4u * (v >> 5), __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, v));
-}
-// (The test is made on the word's address, so up to 31 bits past `end` may be
+// A candidate given as bit index v = 8 * byte + class of the segment at shared
+// address seg, where it lies below send: its word is v / 32 and its mask
+// 0xFFFFFFFE rotated by v (a funnel shift takes its count mod 32).  The test is
+// made on the word's address, so up to 31 bits past the segment's end may be
 // cleared: send is the address past the last word, whose spare bits are masked
-// when it is scanned.)
+// when it is scanned.
 __device__ __forceinline__ void clear_bit_below(uint32_t seg, uint32_t v, uint32_t send) {
   const uint32_t a = seg + 4u * (v >> 5), m = __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, v);
   asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.u32 p, %0, %2;\n\t@p red.shared.and.b32 [%0], %1;\n\t}"
@@ -588,8 +585,9 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
     //    then 32 primes each up to the wheel tier: lanes = (prime q of 4, class
     //      o), eight rounds of four primes, loads of all rounds issued before
     //      any marking so their latency overlaps;
-    //    then 64 primes of one class mod 30 each (the wheel tier, two per
-    //      lane), then kBucketUnit entries of the segment's bucket list each.
+    //    then 2^wlog primes of one class mod 30 each (the wheel tier, one per
+    //      lane at a time), then kBucketUnit entries of the segment's bucket
+    //      list each.
     {
       const uint32_t unp = uniform(np), unb = uniform(nbytes);
       const uint32_t wheel = uniform(S.wheel);
