@@ -138,15 +138,16 @@ struct GapSink {
 
 // Count the gap v - vprev.  Shared bins hold gap/2 < kSmemBins; one extra
 // shared bin (never flushed) absorbs larger gaps, which take the rare path
-// together with a new maximum and gaps >= kLargeGap.
+// together with a new maximum and gaps >= kLargeGap.  The gap starts before any
+// that (maxg, maxgs) stands for (it leads into their run), so it wins a tie.
 __device__ __forceinline__ void record_gap(const GapSink& sk, uint32_t vprev, uint32_t v,
                                            uint32_t& maxg, uint32_t& maxgs) {
   const uint32_t g = v - vprev;
   const uint32_t bin = g >> 1;
   atomicAdd(sk.shist + min(bin, (uint32_t)kSmemBins), 1u);
   // rare: a new maximum or g >= 2 * kSmemBins (which covers g >= kLargeGap)
-  if (g > min(maxg, 2u * (uint32_t)kSmemBins - 1u)) {
-    if (g > maxg) { maxg = g; maxgs = vprev; }
+  if (g >= min(maxg, 2u * (uint32_t)kSmemBins)) {
+    if (g >= maxg) { maxg = g; maxgs = vprev; }
     if (bin >= (uint32_t)kSmemBins)
       atomicAdd(&sk.acc->hist[bin < (uint32_t)kHistBins ? bin : kHistBins - 1], 1ull);
     if (g >= kLargeGap) {
