@@ -125,8 +125,11 @@ int voss_gb300_set_config(const voss_gb300_config_t* cfg);
 /* Offset-regime tuning table (written by voss_gb300/autotune.py, a built-in
  * copy ships in the library): a range [a, b) uses the first entry with
  * b <= b_max and b - a <= width_max.  n = 0 clears the table (the built-in
- * rule then applies).  Bucket lists are used for ranges of 2 to 4096
- * segments. */
+ * rule then applies).  Bucket lists are used for ranges of 2 or more segments
+ * (in a batch or server request, of 2 to 4096).  A caller's table is followed
+ * as it stands; under the built-in one, a lone range of at most a wave of
+ * segments (one per SM) takes lists only where sieving without them, with the
+ * primes of a segment split over several SMs, is measured to be slower. */
 typedef struct {
     uint64_t b_max;
     uint64_t width_max;

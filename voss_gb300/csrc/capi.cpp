@@ -729,10 +729,11 @@ extern "C" int voss_gb300_set_tuning(uint32_t n, const voss_gb300_tune_entry_t* 
     vg::Engine& E = vg::Engine::for_current_device();
     std::lock_guard<std::mutex> g(E.mu);
     if (E.servers) throw vg::Error(VOSS_ERR_INVALID_ARG, "a request server is running on this device");
-    E.tuning.clear();
+    std::vector<vg::TuneEntry> table;
     for (uint32_t i = 0; i < n; ++i)
-      E.tuning.push_back(vg::TuneEntry{e[i].b_max, e[i].width_max, e[i].seg_bytes, e[i].tier_split,
-                                       e[i].bucket_split, 0});
+      table.push_back(vg::TuneEntry{e[i].b_max, e[i].width_max, e[i].seg_bytes, e[i].tier_split,
+                                    e[i].bucket_split, 0});
+    E.set_tuning(std::move(table));
     return VOSS_OK;
   }, VOSS_ERR_INTERNAL);
 }

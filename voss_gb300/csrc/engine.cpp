@@ -97,6 +97,14 @@ Engine& Engine::for_current_device() {
   return *engines[dev];
 }
 
+// the offset-regime table, from timings on a GB300
+const std::vector<TuneEntry>& builtin_tuning() {
+  static const std::vector<TuneEntry> table = {
+#include "tune_table.inc"
+  };
+  return table;
+}
+
 void Engine::init() {
   int n = 0;
   cudaError_t e = cudaGetDeviceCount(&n);
@@ -116,12 +124,7 @@ void Engine::init() {
   scratch.eng = this;
   scratch.device = device;
   scratch.timed = false;           // the one-call path reads no kernel times
-  // the offset-regime table measured by voss_gb300/autotune.py on GB300
-  static const TuneEntry kBuiltin[] = {
-#include "tune_table.inc"
-  };
-  for (const TuneEntry& t : kBuiltin)
-    if (t.seg_bytes) tuning.push_back(t);
+  set_tuning(builtin_tuning());
   ensure_table(65536);
 }
 
@@ -836,7 +839,10 @@ bool Engine::solo_start(uint64_t a, uint64_t b, bool gaps, uint32_t* bitmap) {
     slices = std::max<uint64_t>(1, std::min<uint64_t>(ctas / r.nseg, r.nprimes / kSoloSlicePrimes));
   // (runs with a bitmap never take lists)
   const BucketPlan bp = bucket_plan(c, b, r.nprimes, r.nseg, r.seg_bytes);
-  if (bp.cap && !bitmap && (waves || !cfg.auto_tune || (r.nprimes - bp.bucket_idx) / slices > kSoloListPrimes)) return false;
+  // a caller's configuration or table is followed as it stands; the library's
+  // own splits, which plans and batches share, need kSoloListPrimes here
+  const bool own = cfg.auto_tune && own_tuning;
+  if (bp.cap && !bitmap && (waves || !own || (r.nprimes - bp.bucket_idx) / slices > kSoloListPrimes)) return false;
 
   if (!solo.clean) {
     solo.ctl.reserve(sizeof(SoloCtl));

@@ -210,6 +210,12 @@ struct TuneEntry {
   uint32_t bucket_split;   // primes from here on go through bucket lists; 0 = none
   uint32_t pad;
 };
+inline bool operator==(const TuneEntry& x, const TuneEntry& y) {
+  return x.b_max == y.b_max && x.width_max == y.width_max && x.seg_bytes == y.seg_bytes &&
+         x.tier_split == y.tier_split && x.bucket_split == y.bucket_split;
+}
+// The table that ships in the library.
+const std::vector<TuneEntry>& builtin_tuning();
 
 struct BitmapWork;      // goldbach.cu
 
@@ -266,7 +272,9 @@ class Engine {
   // Bucket layout for a range with the given segment size and segment count.
   BucketPlan bucket_plan(const Config& c, uint64_t b, uint32_t nprimes, uint64_t nseg,
                          uint32_t seg_bytes) const;
+  void set_tuning(std::vector<TuneEntry> table) { tuning = std::move(table); own_tuning = tuning == builtin_tuning(); }
   std::vector<TuneEntry> tuning;
+  bool own_tuning = false;      // `tuning` is the library's table, not a caller's
 
   // The device request of [a, b) under configuration c, without its place in
   // a batch or lists.
