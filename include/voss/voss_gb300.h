@@ -174,7 +174,12 @@ int voss_gb300_plan_kernel_ms(voss_gb300_plan* plan, float* sieve_ms, float* fin
  * goldbach_upto.cu:38-43; the reference does not output it).
  * minp: NULL or (N-4)/2+1 entries, minp[(n-4)/2] = p, 0 for a counterexample.
  * hist: NULL or VOSS_GOLDBACH_HIST_BINS entries, hist[p] = number of n.
- * max_minp, sum_minp, n_counterexamples: NULL or outputs. */
+ * max_minp, sum_minp, n_counterexamples: NULL or outputs.
+ * This call, voss_primes_goldbach_test_upto, voss_primes_in_range*,
+ * voss_primes_nth and the Sophie Germain query keep their device buffers for
+ * the next one, at most 256 MB per GPU (larger ones are given back at the end
+ * of the call); a range, batch or list call that runs out of device memory
+ * gives them back and tries again. */
 #define VOSS_GOLDBACH_HIST_BINS 65536
 int voss_primes_goldbach_minp(uint64_t N, uint32_t* minp, uint64_t* hist,
                               uint32_t* max_minp, uint64_t* sum_minp,

@@ -45,8 +45,23 @@ void DevBuf::reserve(size_t n) {
   if (n <= bytes && ptr) return;
   release();
   size_t want = std::max<size_t>(n, 256);
-  check_cuda(cudaMalloc(&ptr, want), "cudaMalloc");
+  const cudaError_t e = cudaMalloc(&ptr, want);
+  if (e != cudaSuccess) {
+    ptr = nullptr;
+    cudaGetLastError();              // reported here, not by the next launch's check
+  }
+  check_cuda(e, "cudaMalloc");
   bytes = want;
+}
+
+void DevBuf::reserve_ahead(size_t n) {
+  if (n <= bytes && ptr) return;
+  try {
+    reserve(n + std::min<size_t>(n / 8, 32u << 20));
+  } catch (const Error& e) {
+    if (e.code != VOSS_ERR_OUT_OF_MEMORY) throw;
+    reserve(n);
+  }
 }
 
 void DevBuf::release() {
@@ -61,7 +76,12 @@ void HostPinned::reserve(size_t n) {
   ptr = nullptr;
   bytes = 0;
   size_t want = std::max<size_t>(n, 256);
-  check_cuda(cudaMallocHost(&ptr, want), "cudaMallocHost");
+  const cudaError_t e = cudaMallocHost(&ptr, want);
+  if (e != cudaSuccess) {
+    ptr = nullptr;
+    cudaGetLastError();
+  }
+  check_cuda(e, "cudaMallocHost");
   bytes = want;
 }
 
@@ -902,6 +922,11 @@ const ReqResult* Engine::run_solo(uint64_t a, uint64_t b, std::vector<LargeGapRe
 
 const ReqResult* Engine::run(uint32_t n, const uint64_t* a, const uint64_t* b,
                              std::vector<LargeGapRec>* lg, bool gaps, bool share) {
+  return with_room(bitmap_work, [&] { return run_ranges(n, a, b, lg, gaps, share); });
+}
+
+const ReqResult* Engine::run_ranges(uint32_t n, const uint64_t* a, const uint64_t* b,
+                                    std::vector<LargeGapRec>* lg, bool gaps, bool share) {
   if (n == 1)
     if (const ReqResult* r = run_solo(a[0], b[0], lg, gaps)) return r;
   std::vector<uint32_t> rf(n, gaps ? kReqGaps : 0u);

@@ -35,8 +35,9 @@ struct DevBuf {
   size_t bytes = 0;
   void reserve(size_t n);
   // reserve(n) with room for somewhat larger sizes to come (an eighth, at most
-  // 32 MB), for buffers whose size follows a caller's range.
-  void reserve_ahead(size_t n) { if (n > bytes || !ptr) reserve(n + std::min<size_t>(n / 8, 32u << 20)); }
+  // 32 MB) where the device has that room, for buffers whose size follows a
+  // caller's range.
+  void reserve_ahead(size_t n);
   void release();
   template <class T> T* as() const { return static_cast<T*>(ptr); }
   ~DevBuf() { release(); }
@@ -219,6 +220,20 @@ const std::vector<TuneEntry>& builtin_tuning();
 
 struct BitmapWork;      // goldbach.cu
 
+// f(), and where that runs out of device memory while `kept` holds buffers of
+// earlier calls, f() again without them.
+template <class Kept, class F>
+auto with_room(std::shared_ptr<Kept>& kept, F&& f) -> decltype(f()) {
+  const bool held = kept != nullptr;
+  try {
+    return f();
+  } catch (const Error& e) {
+    if (e.code != VOSS_ERR_OUT_OF_MEMORY || !held) throw;
+  }
+  kept.reset();
+  return f();
+}
+
 class Engine {
  public:
   static Engine& for_current_device();
@@ -299,6 +314,8 @@ class Engine {
   Engine() = default;
   void init();
   void build_tiles();
+  const ReqResult* run_ranges(uint32_t n, const uint64_t* a, const uint64_t* b,
+                              std::vector<LargeGapRec>* large, bool gaps, bool share);
   const ReqResult* run_solo(uint64_t a, uint64_t b, std::vector<LargeGapRec>* large, bool gaps);
 };
 

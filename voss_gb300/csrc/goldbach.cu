@@ -561,7 +561,8 @@ GoldbachPlan* goldbach_plan_create(Engine& E, uint64_t N) {
 // What the synchronous calls keep on the device between them: a call that
 // allocates and frees its bitmap pays more for that than for its kernels
 // (Goldbach to 10^9: 0.6 of 2.3 ms; Sophie Germain to 10^7: most of 0.1 ms).
-// Above kKeepBytes everything is given back at the end of the call.
+// Above kKeepBytes everything is given back at the end of the call, and what is
+// kept goes where a call of this engine runs out of device memory (with_room).
 constexpr size_t kKeepBytes = 256u << 20;
 
 struct BitmapWork {
@@ -671,8 +672,8 @@ uint64_t goldbach_plan_probes(GoldbachPlan* g) {
 
 void goldbach_plan_free(GoldbachPlan* g) { delete g; }
 
-GoldbachResult goldbach_run(Engine& E, uint64_t N, uint32_t* minp_host, uint64_t max_ce,
-                            float* kernel_ms) {
+static GoldbachResult goldbach_call(Engine& E, uint64_t N, uint32_t* minp_host, uint64_t max_ce,
+                                    float* kernel_ms) {
   KeptWork work(E);
   GoldbachPlan* const g = &work->gb;
   goldbach_plan_set(g, E, N);
@@ -706,7 +707,12 @@ GoldbachResult goldbach_run(Engine& E, uint64_t N, uint32_t* minp_host, uint64_t
   return r;
 }
 
-uint64_t sophie_germain_count(Engine& E, uint64_t N) {
+GoldbachResult goldbach_run(Engine& E, uint64_t N, uint32_t* minp_host, uint64_t max_ce,
+                            float* kernel_ms) {
+  return with_room(E.bitmap_work, [&] { return goldbach_call(E, N, minp_host, max_ce, kernel_ms); });
+}
+
+static uint64_t sophie_germain_call(Engine& E, uint64_t N) {
   uint64_t seeds = (N >= 2) + (N >= 3) + (N >= 5);
   if (N < 11) return seeds;
   KeptWork work(E);
@@ -725,14 +731,25 @@ uint64_t sophie_germain_count(Engine& E, uint64_t N) {
   return seeds + c;
 }
 
+uint64_t sophie_germain_count(Engine& E, uint64_t N) {
+  return with_room(E.bitmap_work, [&] { return sophie_germain_call(E, N); });
+}
+
 // Ranges up to this width (72 MB of bitmap) are counted by the run that makes
 // their bitmap, unless they surely hold more than max_count primes; others are
 // counted first, so that an oversized request fails before any bitmap is built.
 constexpr uint64_t kOnePassWidth = 1ull << 31;
-constexpr uint64_t kExMaxOnePass = 1024;       // blocks whose offsets the blocks add up themselves (5 * 10^8 wide)
 constexpr uint64_t kExHostRoom = 65536;        // primes of a list that the kernel writes to host memory
+// Room on the device for a list whose length is not known yet (1.79 * 10^8 wide).
+// The bound 2 w / ln w is 2 to 3.5 times what a window holds, so longer lists
+// wait for their count and take what they need.  The wait costs 17 us; of a list
+// of 45 MB, into fresh host pages, that is less than 1% (3 * 10^8 wide at 10^12:
+// 4.4 ms with room for all, 3.8 with a wait and what is needed, which stays kept),
+// but of one whose host pages are there 4% (1.65 * 10^8 wide at 9 * 10^13: 476 us
+// without the wait, 493 with it).
+constexpr uint64_t kExRoomBytes = 144u << 20;
 
-PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count) {
+static PrimeList list_primes(Engine& E, uint64_t a, uint64_t b, uint64_t max_count) {
   PrimeList out;
   std::vector<uint64_t> seeds;
   for (uint64_t q : {2ull, 3ull, 5ull}) if (q >= a && q <= b) seeds.push_back(q);
@@ -759,14 +776,22 @@ PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count)
   const uint32_t* wb = sieve_bitmap(E, work->sieve, a, b + 1, &nw, &solo);
   const uint64_t nblocks = (nw + kExBlockWords - 1) / kExBlockWords;
   work->counts.reserve_ahead(4 * std::max<uint64_t>(nblocks, 1));
-  if (solo && nblocks <= kExMaxOnePass) {
-    // no wait between count and list: the room is what w integers can hold at
-    // most (2 w / ln w primes), a short list goes straight to host memory
-    const double w = (double)(bb - aa) + 2.0;
-    const uint64_t room = std::min<uint64_t>(32 * nw, (uint64_t)(2.0 * w / std::log(w)) + 64);
-    const bool here = room <= kExHostRoom;
-    if (here) work->listed.reserve(8 * kExHostRoom);
-    else work->primes.reserve_ahead(8 * room);
+  // no wait between count and list: the room is what w integers can hold at
+  // most (2 w / ln w primes), a short list goes straight to host memory
+  const double w = (double)(bb - aa) + 2.0;
+  const uint64_t room = std::min<uint64_t>(32 * nw, (uint64_t)(2.0 * w / std::log(w)) + 64);
+  const bool here = room <= kExHostRoom;
+  bool one_pass = solo && 8 * room <= kExRoomBytes;
+  if (one_pass && here) work->listed.reserve(8 * kExHostRoom);
+  if (one_pass && !here) {
+    try {
+      work->primes.reserve_ahead(8 * room);
+    } catch (const Error& e) {
+      if (e.code != VOSS_ERR_OUT_OF_MEMORY) throw;
+      one_pass = false;                      // the list itself may fit
+    }
+  }
+  if (one_pass) {
     uint64_t* const dst = here ? static_cast<uint64_t*>(work->listed.ptr) : work->primes.as<uint64_t>();
     extract_count_kernel<<<(unsigned)nblocks, kExThreads, 0, E.stream>>>(wb, nw, work->counts.as<uint32_t>());
     check_cuda(cudaGetLastError(), "extract_count_kernel");
@@ -806,6 +831,10 @@ PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count)
              "primes");
   check_cuda(cudaStreamSynchronize(E.stream), "in_range");
   return out;
+}
+
+PrimeList primes_in_range(Engine& E, uint64_t a, uint64_t b, uint64_t max_count) {
+  return with_room(E.bitmap_work, [&] { return list_primes(E, a, b, max_count); });
 }
 
 }  // namespace vg
