@@ -135,6 +135,7 @@ void Engine::init() {
   // room for the sieve kernel's dynamic shared memory: the opt-in limit
   // less the kernel's own static shared memory
   max_smem_optin = prop.sharedMemPerBlockOptin - sieve_static_smem_bytes();
+  check_cuda(bucket_fill_ctas_per_sm(&fill_ctas_per_sm), "fill occupancy");
   name = prop.name;
   check_cuda(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
   // Fit the default segment into what this device offers.
@@ -390,7 +391,7 @@ uint32_t Plan::kernels_per_run() const {
 }
 
 uint32_t Plan::fill_grid_max() const {
-  return eng->sm_count * bucket_fill_ctas_per_sm();
+  return eng->sm_count * eng->fill_ctas_per_sm;
 }
 
 bool Plan::overflowed() const {

@@ -241,6 +241,7 @@ class Engine {
   std::mutex mu;     // one caller at a time per device
   int device = 0;
   uint32_t sm_count = 0;
+  uint32_t fill_ctas_per_sm = 1;
   size_t max_smem_optin = 0;    // dynamic shared memory the sieve kernel may ask for
   std::string name;
   cudaStream_t stream = nullptr;
@@ -339,7 +340,7 @@ cudaError_t launch_sieve(const SieveParams& prm, uint32_t grid, uint32_t threads
 cudaError_t launch_solo(const SieveParams& prm, uint32_t threads, cudaStream_t stream);
 cudaError_t launch_lone(const SieveParams& prm, uint32_t grid, uint32_t threads, cudaStream_t stream);
 cudaError_t launch_bucket_fill(const FillParams& fp, uint32_t grid, cudaStream_t stream);
-uint32_t bucket_fill_ctas_per_sm();      // resident fill CTAs per SM (occupancy query, cached)
+cudaError_t bucket_fill_ctas_per_sm(uint32_t* out);      // resident fill CTAs per SM of the current device
 // Cut a batch's ranges at every endpoint into the disjoint pieces some range
 // covers (ascending); a piece gets kReqGaps if a range over it asks for gaps
 // (rflags NULL: all do).  spans[i] = the pieces [s, e) that tile range i.

@@ -1516,14 +1516,14 @@ static cudaError_t fill_attributes() {
   });
 }
 
-uint32_t bucket_fill_ctas_per_sm() {
-  static int n = 0;
-  if (!n && (fill_attributes() != cudaSuccess ||
-             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bucket_fill_kernel, kFillPrimes, sizeof(FillShared)) !=
-                 cudaSuccess ||
-             n < 1))
-    n = 1;
-  return (uint32_t)n;
+cudaError_t bucket_fill_ctas_per_sm(uint32_t* out) {
+  if (cudaError_t e = fill_attributes()) return e;
+  int n = 0;
+  if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bucket_fill_kernel, kFillPrimes,
+                                                                    sizeof(FillShared)))
+    return e;
+  *out = n < 1 ? 1u : (uint32_t)n;
+  return cudaSuccess;
 }
 
 cudaError_t launch_bucket_fill(const FillParams& fp, uint32_t grid, cudaStream_t stream) {
