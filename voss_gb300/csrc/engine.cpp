@@ -838,11 +838,16 @@ constexpr uint64_t kSoloMergeBytes = 4u << 20;
 // width 10^4 at 10^9: 34.8 / 30.3 / 30.7 us with 2048 / 512 / 128; Context(10^7)
 // 38.7 / 38.9 / 37.3).
 constexpr uint32_t kSoloSlicePrimes = 256;
-// Above this many primes per CTA past the bucket split, lists are cheaper: a
-// call of width 10^7 at 9*10^13 (92 000 per CTA) takes 75 us without and 113
-// with them, of 10^8 at 10^12 (59 000) 84 and 92; of 10^8 at 9*10^13 (610 000)
-// the fill is far cheaper.
-constexpr uint32_t kSoloListPrimes = 100000;
+// Above this many primes per CTA past the bucket split, lists are cheaper: where
+// one CTA takes a segment's primes, and where several share them (they share the
+// smaller primes too).  Calls in us without / with lists, width at offset (primes
+// per CTA): one CTA, 5*10^7 at 2*10^12 (88 000) 72 / 76, at 4*10^12 (129 000)
+// 86 / 79, at 9*10^12 (197 000) 102 / 89; several, 2.5*10^7 at 1.1*10^13 (109 000)
+// 72 / 80, at 2*10^13 (147 000) 85 / 90, 2*10^7 at 7*10^13 (181 000) 90 / 95,
+// 2.5*10^7 at 4*10^13 (207 000) 96 / 93, at 7*10^13 (272 000) 111 / 96.  (Beyond
+// 10^8 one CTA's line lies at about 140 000 to 210 000, and the calls on either
+// side of it differ by at most 11%: 3*10^8 at 1.1*10^13, 136 000, 142 / 150.)
+constexpr uint32_t kSoloListPrimes = 100000, kSoloListPrimesShared = 190000;
 constexpr uint32_t kSoloLargeCap = 1u << 14;
 // Segments of a lone_kernel run: 8 MB of records, ranges up to 1.7 * 10^12 wide.
 constexpr uint64_t kLoneMaxSegs = 1u << 18;
@@ -861,9 +866,10 @@ bool Engine::solo_start(uint64_t a, uint64_t b, bool gaps, uint32_t* bitmap) {
   // (runs with a bitmap never take lists)
   const BucketPlan bp = bucket_plan(c, b, r.nprimes, r.nseg, r.seg_bytes);
   // a caller's configuration or table is followed as it stands; the library's
-  // own splits, which plans and batches share, need kSoloListPrimes here
+  // own splits, which plans and batches share, need this many primes here
   const bool own = cfg.auto_tune && own_tuning;
-  if (bp.cap && !bitmap && (waves || !own || (r.nprimes - bp.bucket_idx) / slices > kSoloListPrimes)) return false;
+  const uint32_t pay = slices > 1 ? kSoloListPrimesShared : kSoloListPrimes;
+  if (bp.cap && !bitmap && (waves || !own || (r.nprimes - bp.bucket_idx) / slices > pay)) return false;
 
   if (!solo.clean) {
     solo.ctl.reserve(sizeof(SoloCtl));
