@@ -15,6 +15,7 @@
 #include "engine.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <memory>
 #include <numeric>
@@ -33,12 +34,11 @@ void check_cuda(cudaError_t e, const char* what) {
 }
 
 uint64_t isqrt_u64(uint64_t x) {
-  uint64_t lo = 0, hi = 1ull << 32;
-  while (lo < hi) {
-    const uint64_t mid = lo + (hi - lo + 1) / 2;
-    if (mid <= x / mid) lo = mid; else hi = mid - 1;
-  }
-  return lo;
+  // the double's root is off by one at most
+  uint64_t r = std::min<uint64_t>((uint64_t)std::sqrt((double)x), UINT32_MAX);
+  if (r * r > x) --r;
+  else if (r < UINT32_MAX && (r + 1) * (r + 1) <= x) ++r;
+  return r;
 }
 
 void DevBuf::reserve(size_t n) {
@@ -288,18 +288,26 @@ Config Engine::tuned_for(uint64_t a, uint64_t b, bool batch) const {
     }
   }
   // Alone, a range should fill the GPU in whole waves: the segment shrinks
-  // until the segments come in full waves of one CTA per SM (not below 16 KiB,
-  // where the per-prime setup dominates; with at most 3400 sieving primes not
-  // below 4 KiB: a call over [0, 10^7) takes 34.5 us there, 38.9 with 16 KiB,
-  // one of width 10^7 at 10^12 73 and 43).  In a batch other ranges fill the
-  // GPU, so the largest segment is the cheapest.
+  // until the segments come in full waves of one CTA per SM: not below 4 KiB
+  // with at most 3400 sieving primes (up to 10^9) or with at most 2800 for each
+  // SM to set up, the segments' primes being split over the SMs; not below 16 KiB
+  // elsewhere, where that setup dominates, nor where one segment of up to 8 KiB
+  // covers the range (a call 1.3*10^5 wide below 9*10^8 takes 25.9 us, in two
+  // segments 27.3).  Calls in us with 4 / 16 KiB, width below b (primes per SM):
+  // 10^7 below 9*10^8 (1800) 31 / 33, 5*10^7 (3300) 35 / 36; 10^6 below 1.1*10^9
+  // (210) 28 / 32, 5*10^6 below 10^10 (2600) 31 / 33, 5*10^5 below 10^12 (2600)
+  // 28 / 30; 10^7 below 3*10^9 (3000) 34 / 33, 5*10^6 below 10^11 (7400) 32 / 32,
+  // 10^7 below 10^12 (42 000) 55 / 36.  In a batch other ranges fill the GPU, so
+  // the largest segment is the cheapest.
   if (batch) {
     s = cfg.seg_bytes;
   } else {
     const uint64_t g = (uint64_t)sm_count * cfg.ctas_per_sm;
     const uint64_t waves = (bytes + g * s - 1) / (g * s);
     uint64_t want = (bytes + waves * g - 1) / (waves * g);
-    want = std::max<uint64_t>(want, b <= 1000000000ull ? 4096 : 16384);
+    const uint64_t narrow = std::min<uint64_t>(g, (bytes + 4095) / 4096);     // segments of 4 KiB
+    const bool small = bytes > 8192 && (b <= 1000000000ull || primes_below_sq(b) * narrow <= 2800 * g);
+    want = std::max<uint64_t>(want, small ? 4096 : 16384);
     s = (uint32_t)std::min<uint64_t>(s, (want + 127) & ~127ull);
   }
   c.seg_bytes = s;
