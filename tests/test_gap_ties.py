@@ -26,7 +26,7 @@ def test_random_narrow_windows(vg, oracle_lib):
     for _ in range(4000):
         a = int(rng.integers(0, 2 * 10**7))
         ranges.append((a, a + int(rng.integers(60, 1000 if rng.random() < 0.75 else 4000))))
-    want = [oracle_lib.range_stats(a, b, threads=1) for a, b in ranges]
+    want = [oracle_lib.range_stats(a, b) for a, b in ranges]
     # one by one, a CTA or a few for each; and in batches, cut where they overlap
     for (a, b), orc in zip(ranges, want):
         st = vg.range_stats(a, b)
