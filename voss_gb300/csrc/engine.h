@@ -221,7 +221,7 @@ const std::vector<TuneEntry>& builtin_tuning();
 struct BitmapWork;      // goldbach.cu
 
 // f(), and where that runs out of device memory while `kept` holds buffers of
-// earlier calls, f() again without them.
+// earlier calls, f() again without them (no caller of f uses them meanwhile).
 template <class Kept, class F>
 auto with_room(std::shared_ptr<Kept>& kept, F&& f) -> decltype(f()) {
   const bool held = kept != nullptr;

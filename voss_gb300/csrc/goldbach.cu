@@ -108,7 +108,7 @@ constexpr uint32_t kGbTile = kGbThreads * kGbWords * 32;     // even n per tile
 constexpr uint32_t kGbSmemHist = 4096;                       // p < 4096 counted in smem
 constexpr size_t kGbSmemBytes = kGbSmemHist * 4;
 // The dense bit-set walk stops once at most this many n of a tile are open;
-// the rest are tested a warp per n.
+// the rest are tested by eight lanes per n.
 constexpr uint32_t kGbList = 256;
 // Zero words before and after the odd-number bitmap: a thread's window words
 // (floor(base/32) + kGbWords*tid .. + kGbWords) then never leave the buffer,
@@ -138,9 +138,9 @@ __device__ __forceinline__ uint32_t open_bits(const uint32_t (&U)[kGbWords]) {
 }
 
 // kMinp: write the smallest p of every n (out.minp).  Six blocks per SM (40
-// registers) hide the sparse phase of one behind the walk of the others: 0.76
-// ms at N = 10^9 for the whole plan then, 0.82 with four; 1.64 before the
-// window words stayed in registers and the blocks summed their totals.
+// registers) hide the sparse phase of one behind the walk of the others: the
+// whole plan to N = 10^9 takes 0.687 ms, with five blocks 0.705, and with four it
+// took 0.82 where six took 0.76.
 template <bool kMinp>
 __global__ void __launch_bounds__(kGbThreads, 6)
 goldbach_minp_kernel(const uint32_t* __restrict__ odd,
@@ -179,10 +179,9 @@ goldbach_minp_kernel(const uint32_t* __restrict__ odd,
     // partner n - p is odd bit m - h + 32*(kGbWords*tid + q) + j with m = n0 / 2
     // and h = (p + 1) / 2, so the thread's windows are consecutive bitmap words
     // shifted by (m - h) mod 32.  They stay in registers: m - h moves on by one
-    // word per 64 of p (five times over the first 60 primes).  Loaded for each
-    // prime, at a lane stride of kGbWords words, they took 72 L1 wavefronts
-    // per warp and prime and 0.8 of the kernel's 1.4 ms at N = 10^9; now issue
-    // bounds the walk.
+    // word per 64 of p (five times over the first 60 primes).  So issue bounds
+    // the walk; loaded for each prime, at a lane stride of kGbWords words, they
+    // cost 72 L1 wavefronts per warp and prime, 0.8 ms at N = 10^9.
     uint32_t a[kGbWords + 1];
     const uint64_t m = n0 >> 1;
     const uint32_t* const wp0 = odd + ((m >> 5) + kGbWords * tid);
@@ -235,7 +234,7 @@ goldbach_minp_kernel(const uint32_t* __restrict__ odd,
         U[q] &= ~w;
       }
       // the n resolved at p, per warp: one histogram update (from the bits that
-      // are left, which need no word of hits: 0.724 -> 0.687 ms at N = 10^9)
+      // are left: counting a word of hits instead takes 0.724 ms at N = 10^9)
       const uint32_t now = open_bits(U);
       const uint32_t wres = __reduce_add_sync(0xFFFFFFFFu, left - now);
       left = now;

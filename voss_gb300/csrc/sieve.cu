@@ -664,20 +664,20 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
           // i steps is p (u + i) mod 32, so the lanes, in the order of their u,
           // skip to u + rot = rank + shift, the shift being the least that
           // makes every rot >= 0: 3 steps on average, the longest of a warp
-          // about 6 (a fixed bank per lane took 16 and 31).  A lane walks steps
+          // about 6 (to a fixed bank per lane: 16 and 31).  A lane walks steps
           // rot .. n-1, then wraps to 0 .. rot-1 (wrapped lanes may meet
           // another lane on a bank, and test for their wrap at each step).
-          // [0, 10^10): 1.074 -> 1.042 ms, and as the primes with few steps
-          // gain most, the split to the mid tier moved from 1400..1700 to 2048
-          // (1.042 -> 1.039; [10^12, 1.01*10^12) 1.435 -> 1.408 -> 1.390).
+          // [0, 10^10) takes 1.042 ms with the order and 1.074 with fixed
+          // banks; with it the tier pays up to 2048 (1.039 ms, up to 1400..1700
+          // 1.042; [10^12, 1.01*10^12) 1.390 and 1.408).
           const uint32_t j0 = s + h * p;
           const uint32_t c = j0 & 3u;
           const uint32_t mask = ~(1u << ((c << 3) | o));
           const uint32_t lim = (unb - c + 3u) >> 2;         // word w holds byte 4w + c < nbytes
           const uint32_t w0 = j0 >> 2;
-          // steps: w0 < p, so floor(whole words / p) or one more (the floor by
-          // a multiplication, exact for factors below 2^16; with a division, a
-          // remainder and two reductions [0, 10^10) took 1.037 ms, now 1.033)
+          // steps: w0 < p, so floor(whole words / p) or one more, the floor by a
+          // multiplication, exact for factors below 2^16 ([0, 10^10) 1.033 ms;
+          // with a division, a remainder and two reductions 1.037)
           const uint32_t nmin = __umulhi(unb >> 2, minv);
           const uint32_t n = nmin + (w0 + nmin * p < lim ? 1u : 0u);
           const uint32_t pinv = p * (2u - p * p);           // p^-1 mod 64 (p odd, p*p = 1 mod 8)
@@ -727,14 +727,13 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
           // wheel tier: a lane per prime of one class mod 30, its eight hits
           // per turn of p bytes in the order of their cofactors w mod 30: the
           // first lies at t w + const - k0 (mod p), the next ones follow by p.
-          // With the eight residues of each prime read from memory (44 bytes
-          // where this takes 8, as many shared-memory wavefronts as the
-          // clears), a 64-bit reduction and a branch per clear, the primes
-          // above the segment took 168 instructions per prime and segment and
-          // those below it 13 per clear; now about 100 (60 from 2.5 segments
-          // on) and 6.  [9*10^11, 10^12): 20.8 -> 16.5 ms with the uniform
-          // unit bounds.  What bounds it: shared-memory wavefronts (3.5 per
-          // atomic on random banks) below the segment size, issue above.
+          // What bounds it: shared-memory wavefronts (3.5 per atomic on random
+          // banks) below the segment size, at 6 instructions per clear; issue
+          // above, at about 100 instructions per prime and segment, 60 from 2.5
+          // segments on.  Reading a prime's eight residues instead costs 44
+          // bytes where this takes 8, and with a 64-bit reduction and a branch
+          // per clear 168 and 13 instructions ([9*10^11, 10^12) 20.8 ms to 16.5
+          // when that was the difference).
           const uint32_t wu = u - nsmall - nmidu;
           const uint32_t cls = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, lane < 8u && wu >= wincl));
           const uint32_t ubeg = __shfl_sync(0xFFFFFFFFu, wincl, (cls + 31u) & 31u);
@@ -752,9 +751,9 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
           if (pfirst >= 15u * unb) {
             // at most one hit at all (cofactors coprime to 30 lie 2 apart or
             // more): the first multiple p (30 a + w) of the segment is found
-            // directly, from 30 (k0 mod p) / p and the next w from there.  (As
-            // the smallest of the eight classes' hits, below, a prime took 40
-            // operations on the integer pipe, twice its share; here 16.)
+            // directly, from 30 (k0 mod p) / p and the next w from there: 16
+            // operations on the integer pipe (as the smallest of the eight
+            // classes' hits, below, 40, twice its share).
             constexpr uint32_t kCoprime = 0xA08A2882u;    // residues 1 7 11 13 17 19 23 29, and 31 for the next turn's 1
             auto mark = [&](uint2 q) {
               const uint32_t p = 30u * q.x + cc, inv = q.y;
@@ -879,7 +878,7 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
             const uint32_t m = __shfl_sync(0xFFFFFFFFu, mm, 4 * t + h);
             uint32_t s = rr[t] - m;
             s = min(s, s + p);
-              const bool mine = (lane >> 2) == (uint32_t)t;
+            const bool mine = (lane >> 2) == (uint32_t)t;
             const uint32_t nall = __reduce_min_sync(0xFFFFFFFFu, mine ? nm : ~0u);
             const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, mine ? nm : 0u) + 1u;
             uint32_t j = sseg + s, k = 0;
@@ -959,9 +958,9 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
         // previous prime in the gap histogram, and the largest such gap is
         // kept as g << 23 | (2^23 - 1 - end), the earliest first on ties
         // (nv and npv are 2^23 - 1 - the gap's end and start).
-        // (Before, a 16-byte table entry per byte brought the inner gaps as
-        // packed counters: 12 shared-memory wavefronts and 35 instructions
-        // per byte and warp, now 7 and 24: [9*10^11, 10^12) 16.5 -> 14.8 ms.)
+        // 7 shared-memory wavefronts and 24 instructions per byte and warp,
+        // and issue bounds it (a 16-byte table entry per byte with the inner
+        // gaps as packed counters: 12 and 35, [9*10^11, 10^12) 16.5 ms to 14.8).
         // A run is walked prime by prime only where it holds a gap beyond the
         // shared bins, or where no gap between bytes of the whole warp exceeds
         // 28, the largest inside a byte.
@@ -1013,8 +1012,9 @@ __device__ __forceinline__ void sieve_body(const SieveParams& prm) {
       } else {
         // Count only: the run's words are added bit by bit (carry-save, eight
         // words per step), so three masked popcounts per step of eight words
-        // give the primes and those 1 mod 4 and 1 mod 3; popcounts (a quarter
-        // of the integer rate) of every word took most of the scan.
+        // give the primes and those 1 mod 4 and 1 mod 3; popcounts run at a
+        // quarter of the integer rate (of every word, a count to 3*10^10 takes
+        // 2.83 ms to 2.71).
         uint32_t ones = 0, twos = 0, fours = 0, n8 = 0, a8 = 0, b8 = 0;
         constexpr uint32_t m31 = 0x2B2B2B2Bu;
         auto add = [](uint32_t& s, uint32_t x, uint32_t y) {      // s + x + y per bit: the sum, and the carry
@@ -1175,11 +1175,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) solo_kernel(const __grid_const
 
 // A lone request of more segments than a wave, without lists, in one launch:
 // one CTA per SM takes segments from a queue, and the last CTA to find it empty
-// writes the result to host memory.  As a plan the same request took a copy up,
+// writes the result to host memory.  As a plan the same request takes a copy up,
 // a zeroing launch, the sieve, a launch of one block that folds the records
-// and two copies down with a wait each: Context(10^10) 1079 -> 1052 us, 2*10^9
-// numbers at 0 234 -> 221, Context(10^12) 125.5 -> 124.3 ms (one block folded
-// its 150 000 records).
+// and two copies down with a wait each: Context(10^10) 1079 us instead of 1052,
+// 2*10^9 numbers at 0 234 instead of 221, Context(10^12) 125.5 ms instead of
+// 124.3.
 __global__ void __launch_bounds__(kMaxThreads, 1) lone_kernel(const __grid_constant__ SieveParams prm) {
   sieve_body<kFormLone>(prm);
 }
@@ -1189,8 +1189,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) lone_count_kernel(const __grid
   sieve_body<kFormLoneCount>(prm);
 }
 
-// A CTA per request; a lone one's records are folded by 1024 threads instead of
-// 256 (150 000 records: 0.54 -> 0.18 ms).
+// A CTA per request; a lone one's records are folded by 1024 threads (150 000
+// records: 0.18 ms, by 256 threads 0.54).
 __global__ void __launch_bounds__(kMaxThreads)
 finalize_kernel(const ReqDesc* __restrict__ reqs, const BatchHdr* __restrict__ hdr,
                 const SegRec* __restrict__ segs, ReqAccum* __restrict__ acc, LargeGapRec* large,
@@ -1209,14 +1209,12 @@ finalize_kernel(const ReqDesc* __restrict__ reqs, const BatchHdr* __restrict__ h
 // hit's byte k in the item's segments; its segment is k / S by a
 // multiplication, and its entry goes to the next place of that segment's bin
 // in shared memory.  Then one global atomic per segment reserves room in that
-// segment's list, and a warp per segment copies its bin there.  What bounds
-// it: shared-memory wavefronts and issue, half and half (a returning atomic
-// and a store on random banks per hit).
-// Before, a first walk counted the hits and a second one stored each entry
-// from its lane: 16 write requests per 32 entries (now 3) were the bound, and
-// the chains' segment, offset and count took 23 instructions per hit and walk.
-// [10^14, 10^14 + 10^9): 97 -> 82 us of 342 -> 325; [10^14 - 10^11, 10^14):
-// 26.8 -> 24.4 ms in all.
+// segment's list, and a warp per segment copies its bin there: 3 write requests
+// per 32 entries.  What bounds it: shared-memory wavefronts and issue, half and
+// half (a returning atomic and a store on random banks per hit).
+// [10^14, 10^14 + 10^9) 82 us of 325, [10^14 - 10^11, 10^14) 24.4 ms in all;
+// counting in a first walk and storing each entry from its lane in a second one,
+// with 16 write requests per 32 entries as the bound, 97 of 342 us and 26.8 ms.
 // The bins hold 1.54 times an item's expected hits: with at most kFillSegs
 // segments their mean is 54 entries and the margin 4 standard deviations.
 // Primes near sqrt(b) have their hits in clusters (p q = s^2 / 4 - d^2 / 4

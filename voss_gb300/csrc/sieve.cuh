@@ -139,8 +139,9 @@ inline void build_wheel_table(const uint32_t* P, uint32_t n, WheelEntry* W, uint
 // primes from seg_bytes / kWheelDiv on, not below the warp-per-prime tier
 // (index split) nor kWheelMinPrime.  index_of(p): first table index >= p.
 // Further down a batch of 32 primes of one class spans too wide a range of p:
-// its last turns run half idle ([0, 10^10) 1.313 / 1.319 / 1.335 ms, [9*10^11,
-// 10^12) 17.0 / 16.8 / 16.8 ms with the tier from S/8 / S/16 / S/32 on).
+// its last turns run half idle ([0, 10^10) 1.018 / 1.021 / 1.029 / 1.044 ms,
+// [10^12, 1.01*10^12) 1.383 / 1.373 / 1.380 / 1.413 ms with the tier from S/12 /
+// S/16 / S/24 / S/32 on).
 constexpr uint32_t kWheelDiv = 16;
 template <class IndexOf>
 inline uint32_t wheel_begin_index(uint32_t seg_bytes, uint32_t split, IndexOf index_of) {
